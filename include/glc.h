@@ -234,8 +234,9 @@ glc_status glc_commit_batch_fused_cancellable(const glc_commit_job *jobs, uint32
  * Released with glc_mapped_word_destroy(host). */
 glc_status glc_mapped_word_create(uint32_t **host, uint32_t **device);
 glc_status glc_mapped_word_destroy(uint32_t *host);
-/* Waits of glc_commit_batch_fused that expired on the current device since the library was
- * loaded (0 unless something is wrong; a launch with an expired wait computes wrong results).
+/* Waits of glc_commit_batch_fused, and of NTT kernels for the tensor cores, that expired on the
+ * current device since the library was loaded (0 unless something is wrong; a launch with an expired
+ * wait computes wrong results).
  * Synchronous. */
 glc_status glc_commit_batch_fused_timeouts(uint64_t *out);
 
@@ -297,6 +298,8 @@ glc_status glc_server_destroy(glc_server *server);
  * them (or autotune) before other host threads launch work on that device.  Every choice
  * computes the same bits.
  */
+/* For the NTT passes in registers; batches large enough for the tensor cores (from 2^20 elements, 2^21
+ * on a coset) have a fixed plan. */
 typedef struct glc_ntt_tuning {
   uint32_t radix_bits;       /* stages per register round: 2, 3 or 4 */
   uint32_t k1;               /* stages in the strided pass of a two-pass NTT (0 = log_n / 2) */

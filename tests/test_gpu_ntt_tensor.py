@@ -1,0 +1,62 @@
+"""The NTT passes on the tensor cores against the oracle: every split of the stages into rounds,
+column groups with remainders, in place and out of place, offsets and strides that forbid the wide
+stores, at and just above the sizes from which batches take this path."""
+import numpy as np
+import pytest
+
+from conftest import canon, load_package, rand_elems
+from gpu_util import from_dev, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def glc():
+    g = load_package()
+    ctx = g.Context.create()
+    yield g
+    ctx.destroy()
+
+
+@pytest.mark.parametrize("log_n,cols", [(12, 256), (12, 513), (12, 5000), (16, 16), (16, 67), (17, 16), (18, 8), (19, 5),
+                                        (20, 2), (21, 1), (22, 1), (23, 1), (24, 16)])
+@pytest.mark.parametrize("bitrev,inverse,log_ext,coset", [(False, False, 0, 0), (False, True, 0, 0), (True, False, 0, 0),
+                                                          (True, True, 0, 0), (False, False, 3, 5)])
+def test_against_oracle(glc, oracle, log_n, cols, bitrev, inverse, log_ext, coset):
+    n = 1 << log_n
+    # 12 x 513: odd offset and stride; 16 x 67: even, not a multiple of 4; 24 x 16: too large for two cases
+    off, gap = {(12, 513): (1, 3), (16, 67): (2, 6), (18, 8): (3, 4)}.get((log_n, cols), (0, 0))
+    if log_n == 24 and not (inverse and not bitrev):
+        pytest.skip("one direction at the largest size")
+    stride = n + gap
+    x = rand_elems(cols * stride, log_n * 1000 + cols, noncanonical=True)
+    want = np.full(cols * stride, 7, dtype=np.uint64)
+    packed = np.ascontiguousarray(x.reshape(cols, stride)[:, off:off + n])
+    want.reshape(cols, stride)[:, off:off + n] = oracle.batch_ntt(packed.reshape(-1), log_n, cols, n, n, int(bitrev),
+                                                                  int(inverse), log_ext, coset).reshape(cols, n)
+    src, out = to_dev(x), to_dev(np.full(cols * stride, 7, dtype=np.uint64))
+    glc.ntt.batch_ntt_out_of_place(src, out, log_n, cols, off, off, stride, stride, bitrev, inverse, log_ext, coset)
+    assert (from_dev(src) == x).all()
+    assert (from_dev(out) == want).all()
+    glc.ntt.batch_ntt_in_place(src, log_n, cols, off, stride, bitrev, inverse, log_ext, coset)
+    got = from_dev(src).reshape(cols, stride)
+    assert (got[:, off:off + n] == want.reshape(cols, stride)[:, off:off + n]).all()
+    assert (got[:, :off] == x.reshape(cols, stride)[:, :off]).all()
+    assert (got[:, off + n:] == x.reshape(cols, stride)[:, off + n:]).all()
+    assert glc.commit.fused_timeouts() == 0
+
+
+def test_column_groups_past_the_grid(glc, oracle):
+    """More column groups than one launch's grid holds (65535 groups of 16 columns)."""
+    cols, n = 16 * 65535 + 35, 1 << 12
+    import torch
+    free, _ = torch.cuda.mem_get_info()
+    if free < 40 * cols * n:
+        pytest.skip("needs %d GB" % (40 * cols * n >> 30))
+    x = torch.randint(0, 2**62, (cols, n), device="cuda")
+    keep = [0, 15, 16, 16 * 65535 - 1, 16 * 65535, cols - 1]
+    before = x[keep].cpu().numpy().view(np.uint64)
+    glc.ntt.batch_ntt_in_place(x, 12, cols, 0, n, False, True, 0, 0)
+    got = x[keep].cpu().numpy().view(np.uint64)
+    want = oracle.batch_ntt(np.ascontiguousarray(before).reshape(-1), 12, len(keep), n, n, 0, 1, 0, 0)
+    assert (canon(got.reshape(-1)) == want).all()

@@ -53,6 +53,8 @@ static void free_tables(DeviceTables &t) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
+  if (t.dft) cudaFree(t.dft);
+  t.dft = nullptr;
   t.ready = false;
 }
 
@@ -114,6 +116,7 @@ extern "C" glc_status glc_context_create(uint32_t powers_of_w_coarse_log_count, 
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = (cudaError_t)ntt_init_device();
+  if (e == cudaSuccess) e = (cudaError_t)ntt_dft_create(&t.dft);
   if (e != cudaSuccess) {
     free_tables(t);
     return (int)e;

@@ -606,7 +606,10 @@ extern "C" glc_status glc_mapped_word_destroy(uint32_t *host) { return host ? (i
 extern "C" glc_status glc_commit_batch_fused_timeouts(uint64_t *out) {
   if (!out) return fail("commit_batch_fused_timeouts: null output");
   unsigned long long v = 0;
-  const cudaError_t e = cudaMemcpyFromSymbol(&v, g_fused_timeouts, sizeof(v));
+  cudaError_t e = cudaMemcpyFromSymbol(&v, g_fused_timeouts, sizeof(v));
+  uint64_t ntt = 0;
+  if (e == cudaSuccess) e = (cudaError_t)ntt_expired_waits(&ntt);
+  v += ntt;
   *out = v;
   return (int)e;
 }

@@ -7,9 +7,11 @@
 //    k consecutive radix-2 stages.  Writing a position as i = hi*2^(L-s0) + mid*M + lo
 //    (M = 2^(L-s0-k)), the pass transforms the 2^k values of every (hi, lo) group.  One CTA
 //    owns a tile of W consecutive lo values of one hi (W*8 bytes contiguous per row: coalesced
-//    128-bit loads), stages it in shared memory and runs the k stages as radix-8 register
-//    rounds with XOR-swizzled shared-memory exchanges.  The CTA walks several columns with the
-//    same twiddles, which it builds once in shared memory.
+//    128-bit loads), stages it in shared memory and runs the k stages as radix-4..16 register
+//    rounds with shared-memory exchanges in a padded layout.  The CTA walks several columns with
+//    the same twiddles, which it builds once in shared memory.
+//  * Batches that fill the GPU run their rounds on the tensor cores instead (ntt_tensor.cuh, chosen
+//    by tt_usable): 2^22 x 176 in 10.9 ms where the register rounds take 16.5 ms.
 //  * n2b (natural -> bit-reversed) runs the stages in increasing order with DIT butterflies,
 //    b2n (bit-reversed -> natural) is its transpose: decreasing order, DIF butterflies.  Both
 //    use the twiddle T[b] = w^bitrev(b) of block b at each stage; T is one flat table.
@@ -20,9 +22,11 @@
 //    NTT is integer-bound, and small chunks cost more in per-CTA twiddle tables than they save
 //    in HBM traffic, so the default is one chunk.
 #include <algorithm>
+#include <vector>
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
+#include "ntt_tensor.cuh"
 #include "ntt_tile.cuh"
 
 namespace glc {
@@ -87,6 +91,29 @@ int ntt_init_device() {
   cudaError_t e = cudaFuncSetAttribute(ntt_pass_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, NTT_SMEM_MAX);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(ntt_pass_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, NTT_SMEM_MAX);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(ntt_pass_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, NTT_SMEM_MAX);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(ntt_tensor_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, NTT_SMEM_MAX);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(ntt_tensor_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, NTT_SMEM_MAX);
+  return (int)e;
+}
+
+int ntt_expired_waits(uint64_t *out) {
+  unsigned long long v = 0;
+  const cudaError_t e = cudaMemcpyFromSymbol(&v, d_ntt_expired, sizeof(v));
+  *out = v;
+  return (int)e;
+}
+
+int ntt_dft_create(uint8_t **out) {
+  std::vector<uint8_t> m(4 * DFT_BYTES);
+  for (uint32_t v = 0; v < 4; v++)
+    for (uint32_t r = 2; r <= 4; r++) {
+      uint8_t *p = m.data() + v * DFT_BYTES + dft_offset(r);
+      const uint64_t w16 = h_root_of_unity(4);
+      uint64_t *coefs = reinterpret_cast<uint64_t *>(m.data() + v * DFT_BYTES + DFT_MATRICES + dft_offset(r) / 8);
+      build_dft_matrix(p, coefs, r, v & 1, v & 2 ? h_inv(w16) : w16);
+    }
+  cudaError_t e = cudaMalloc(out, m.size());
+  if (e == cudaSuccess) e = cudaMemcpy(*out, m.data(), m.size(), cudaMemcpyHostToDevice);
   return (int)e;
 }
 
@@ -125,6 +152,20 @@ NttTuning &ntt_tuning(uint32_t log_n) {
   return g_ntt_tuning[(dev >= 0 && dev < MAX_DEVICES) ? dev : 0][std::min(log_n, MAX_LOG_N)];
 }
 
+// Whether a batch runs its passes on the tensor cores (ntt_tensor.cuh).  Needed: whole tiles (2^12
+// rows, or at least 4 strided stages before 12 contiguous ones), and no per-element coset factor
+// (a coset on the b2n side or in an inverse).  Worth it when the tiles fill the GPU, since a tile's
+// rounds are a longer chain of latencies than the small tiles of ntt_pass_kernel, and a coset's
+// matrices and twiddles cost more to build.  Measured on B200, us, tensor cores / radix passes:
+//   no coset: 16 x 2^16 (256 tiles) 30 / 30, 4 x 2^18 33 / 36, 1 x 2^20 34 / 40; 8 x 2^16 (128) 23 / 22
+//   coset:    32 x 2^16 (512 tiles) 47 / 53, 8 x 2^18 52 / 61; 16 x 2^16 (256) 36 / 32, 4 x 2^18 39 / 38
+//   2^24, whose strided rows hold one element: 1 column 636 / 565, 16 columns 7761 / 8482
+static bool tt_usable(uint32_t log_n, uint32_t num_ntts, bool bitrev_inputs, bool inverse, uint32_t log_ext) {
+  if (log_n < TT_LOG || (log_n > TT_LOG && log_n < TT_LOG + 4) || (log_ext && (inverse || bitrev_inputs))) return false;
+  if (log_n == 24 && num_ntts < 16) return false;
+  return ((uint64_t)num_ntts << (log_n - TT_LOG)) >= (log_ext ? 512 : 256);
+}
+
 int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_ntts, uint64_t in_stride,
                uint64_t out_stride, bool bitrev_inputs, bool inverse, uint32_t log_ext, uint32_t coset_idx,
                cudaStream_t stream, uint32_t l2_chunk_cols) {
@@ -134,6 +175,19 @@ int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_n
   const NttTuning &tu = ntt_tuning(log_n);
   Pass passes[2];
   const uint32_t np = make_plan(log_n, bitrev_inputs, tu, passes);
+  if (tt_usable(log_n, num_ntts, bitrev_inputs, inverse, log_ext)) {
+    const uint32_t k0 = log_n - TT_LOG;  // strided stages, then 12 contiguous ones
+    if (k0 == 0)
+      return tt_launch_pass(t, 0, TT_LOG, true, true, in, out, in_stride, out_stride, num_ntts, log_n, bitrev_inputs,
+                            inverse, log_ext, coset_idx, stream);
+    for (uint32_t q = 0; q < 2; q++) {
+      const bool strided = bitrev_inputs ? q == 1 : q == 0;
+      const int e = tt_launch_pass(t, strided ? 0 : k0, strided ? k0 : TT_LOG, q == 0, q == 1, in, out, in_stride, out_stride,
+                                   num_ntts, log_n, bitrev_inputs, inverse, log_ext, coset_idx, stream);
+      if (e) return e;
+    }
+    return 0;
+  }
   const uint64_t n = 1ull << log_n;
   if (l2_chunk_cols == 0) {
     // keep one chunk of columns resident in L2 across the passes
