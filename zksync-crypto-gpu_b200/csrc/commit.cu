@@ -123,7 +123,7 @@ int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *ev
     if (!e) e = mark();
     if (e) return e;
     uint64_t *tree = j.trees + (uint64_t)c * 8 * n;
-    e = p2_leaves_launch(dst, tree, 0, j.cols, n, false, false, cur);
+    e = p2_leaves_launch(dst, tree, 0, j.cols, n, false, false, cur, coset_parallel ? f * n : ~0ull);
     if (!e) e = mark();
     if (e) return e;
     if (layers > 1) {

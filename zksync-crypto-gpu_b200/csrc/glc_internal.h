@@ -80,8 +80,10 @@ int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_n
                cudaStream_t stream, uint32_t l2_chunk_cols);
 int bitrev_launch(const uint64_t *src, uint64_t src_stride, uint64_t *dst, uint64_t dst_stride, uint32_t log_rows,
                   uint32_t cols, cudaStream_t stream);
+// together: leaves that other streams hash at the same time, these included (a launch that shares the
+// GPU takes the form that needs the fewest instructions, not the shortest chain).
 int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t rows, uint64_t cols, uint64_t count,
-                     bool load_intermediate, bool store_intermediate, cudaStream_t stream);
+                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, uint64_t together = 0);
 int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, cudaStream_t stream);
 // Node layers of a tree whose leaf layer ([4][leaves]) starts at `layer0`; writes layers 1..layers
 // into the following part of the same buffer (reference layout, poseidon2.rs:276-314).

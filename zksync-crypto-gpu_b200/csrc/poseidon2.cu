@@ -9,8 +9,9 @@
 //    the next round's constants are added before that reduction, so a round constant costs no
 //    modular addition;
 //  * round constants live in __constant__ memory (uniform across a warp: one broadcast read);
-//  * Merkle node layers run as fused subtrees: one CTA hashes 2*T children down through
-//    log2(2T) layers in shared memory, so a tree of 2^20 leaves needs 3 launches, not 20.
+//  * launches that cannot fill the GPU with one thread per permutation take four lanes per
+//    permutation (p2_spread.cuh), and a tree's narrow layers run as fused subtrees, up to 7 layers a
+//    launch.
 #include <algorithm>
 
 #include "glc_field.cuh"
@@ -296,6 +297,10 @@ __device__ __forceinline__ void permutation(uint64_t s[WIDTH]) {
   for (int i = 0; i < WIDTH; i++) s[i] = canon(s[i]);
 }
 
+}  // namespace glc
+#include "p2_spread.cuh"
+namespace glc {
+
 // Leaf hashes (poseidon2_gl_st.cu:25-59): leaf i absorbs values[(i<<r) + row + col*rows*count]
 // column by column, rows within a column, 8 per permutation into state[0..8) (overwrite),
 // zero-padding the last chunk.  Capacity state[8..12) starts at 0 or is loaded from results.
@@ -395,60 +400,6 @@ __global__ void __launch_bounds__(256) p2_nodes_kernel(const uint64_t *values, u
   for (int k = 0; k < 4; k++) results[k * count + gid] = o[k];
 }
 
-// Fused node layers: the CTA owns 2*T consecutive children of layer `in` ([4][2*count]) and
-// produces up to `layers` parent layers, the j-th written to out_j ([4][count >> j] at
-// out + offset of layer j).  out points at the first parent layer; each following layer starts
-// right after the previous one (reference tree layout, poseidon2.rs:276-314).
-template <uint32_t T, int ROLL, bool LAZY>
-__global__ void __launch_bounds__(T) p2_subtree_kernel(const uint64_t *in, uint64_t *out, uint64_t count,
-                                                       uint32_t layers, bool aligned) {
-  __shared__ uint64_t sh[4][T];
-  const uint32_t tid = threadIdx.x;
-  uint64_t layer_count = count;          // nodes in the layer being produced
-  uint64_t node = (uint64_t)blockIdx.x * T + tid;  // this thread's node in that layer
-  uint64_t *dst = out;
-  uint32_t active = T;
-  // first layer: children straight from global memory
-  {
-    uint64_t l[4], r[4], o[4];
-    const bool live = node < layer_count;
-    if (live) {
-      load_children(in, layer_count, node, l, r, aligned);
-      hash_node<ROLL, LAZY>(l, r, o);
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        dst[k * layer_count + node] = o[k];
-        sh[k][tid] = o[k];
-      }
-    }
-  }
-  for (uint32_t j = 1; j < layers && active > 1; j++) {
-    __syncthreads();
-    dst += 4 * layer_count;
-    layer_count >>= 1;
-    active >>= 1;
-    node = (uint64_t)blockIdx.x * active + tid;
-    uint64_t o[4];
-    const bool live = tid < active && node < layer_count;
-    if (live) {
-      uint64_t l[4], r[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        l[k] = sh[k][2 * tid];
-        r[k] = sh[k][2 * tid + 1];
-      }
-      hash_node<ROLL, LAZY>(l, r, o);
-#pragma unroll
-      for (int k = 0; k < 4; k++) dst[k * layer_count + node] = o[k];
-    }
-    __syncthreads();
-    if (live) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) sh[k][tid] = o[k];
-    }
-  }
-}
-
 // gather_rows (queries.cuh:9-19)
 __global__ void p2_gather_rows_kernel(const uint32_t *indexes, uint32_t indexes_count, uint32_t log_rows_per_index,
                                       const uint64_t *values, uint64_t values_stride, uint64_t *results,
@@ -513,9 +464,29 @@ static void leaves_go(uint32_t minb, uint32_t blocks, uint32_t threads, cudaStre
       F(0, false);                        \
   } while (0)
 
+// Up to HEX_MAX permutations at once take 16 lanes each, up to QUAD_MAX four, more a thread each.
+// Measured on B200, us a launch of one permutation each, 16 lanes / 4 lanes / a thread: 1024 leaves
+// 13.9 / 16.0 / 21.6; 2048: 14.9 / 15.9 / 21.5; 4096: 19.9 / 15.7 / 21.6; 8192: 31.8 / 16.4 / 21.6;
+// 16384: 50 / 25.8 / 21.7.
+static constexpr uint64_t HEX_MAX = 2048, QUAD_MAX = 8192;
+
+static uint32_t spread_grid(uint64_t count, uint32_t lanes) {
+  return (uint32_t)((count * lanes + SPREAD_THREADS - 1) / SPREAD_THREADS);
+}
+
 int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint64_t cols, uint64_t count,
-                     bool load_intermediate, bool store_intermediate, cudaStream_t stream) {
+                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, uint64_t together) {
   if (count == 0) return 0;
+  together = std::max(together, count);
+  if (together <= QUAD_MAX) {
+    if (together <= HEX_MAX)
+      p2_leaves_spread_kernel<16><<<spread_grid(count, 16), SPREAD_THREADS, 0, stream>>>(
+          values, results, log_rows, cols, count, load_intermediate, store_intermediate);
+    else
+      p2_leaves_spread_kernel<4><<<spread_grid(count, 4), SPREAD_THREADS, 0, stream>>>(
+          values, results, log_rows, cols, count, load_intermediate, store_intermediate);
+    return last_launch_error();
+  }
   const P2Tuning &tu = p2_tuning();
   const uint32_t threads = tu.leaf_threads;
   const uint64_t blocks = (count + threads - 1) / threads;
@@ -527,8 +498,21 @@ int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_row
   return last_launch_error();
 }
 
+// Node layers that one spread launch makes, from the first of `count` nodes: a CTA's 64 (quads) or 16
+// nodes down to one.
+static uint32_t spread_layers(uint64_t count) { return count <= HEX_MAX ? 5 : 7; }
+static int p2_subtree_launch(const uint64_t *in, uint64_t *out, uint64_t count, uint32_t layers, cudaStream_t stream) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+  if (count <= HEX_MAX)
+    p2_subtree_spread_kernel<16><<<spread_grid(count, 16), SPREAD_THREADS, 0, stream>>>(in, out, count, layers, aligned);
+  else
+    p2_subtree_spread_kernel<4><<<spread_grid(count, 4), SPREAD_THREADS, 0, stream>>>(in, out, count, layers, aligned);
+  return last_launch_error();
+}
+
 int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, cudaStream_t stream) {
   if (count == 0) return 0;
+  if (count <= QUAD_MAX) return p2_subtree_launch(values, results, count, 1, stream);
   const P2Tuning &tu = p2_tuning();
   const uint32_t threads = tu.leaf_threads;
   const uint64_t blocks = (count + threads - 1) / threads;
@@ -541,43 +525,21 @@ int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, c
 }
 
 int p2_tree_nodes_launch(uint64_t *layer0, uint64_t leaves, uint32_t layers, cudaStream_t stream) {
-  constexpr uint32_t T = 128;
   const uint64_t *in = layer0;
   uint64_t *out = layer0 + 4 * leaves;
   uint64_t count = leaves >> 1;  // nodes of the first layer to produce
-  uint32_t remaining = layers;
-  // Wide layers: one launch per layer keeps every thread busy.  Once a layer no longer fills
-  // the GPU a few times over, fused subtree launches cover up to 8 layers each, so the narrow
-  // top of the tree costs a handful of launches instead of one per layer.
-  const uint64_t wide = 148ull * 128;
-  while (remaining > 0 && count >= wide) {
-    const int e = p2_nodes_launch(in, out, count, stream);
+  // Wide layers: one launch per layer, one thread per node.  Narrower ones, up to 7 in a launch: a
+  // CTA's 64 nodes down to one, four lanes per node.
+  while (layers > 0) {
+    const uint32_t l = count > QUAD_MAX ? 1 : std::min(layers, spread_layers(count));
+    const int e = count > QUAD_MAX ? p2_nodes_launch(in, out, count, stream) : p2_subtree_launch(in, out, count, l, stream);
     if (e) return e;
-    in = out;
-    out += 4 * count;
-    count >>= 1;
-    remaining--;
-  }
-  while (remaining > 0) {
-    // one launch covers up to log2(T)+1 layers (T threads -> 1 node)
-    uint32_t l = 1;
-    while (l < remaining && (T >> l) >= 1 && l < 8) l++;
-    const uint64_t blocks = (count + T - 1) / T;
-    if (blocks > 0x7fffffffull) return fail("poseidon2: too many nodes");
-    const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-    const P2Tuning &tu = p2_tuning();
-#define GLC_SUB(R, L) p2_subtree_kernel<T, R, L><<<(uint32_t)blocks, T, 0, stream>>>(in, out, count, l, aligned)
-    GLC_P2_VARIANT(tu, GLC_SUB);
-#undef GLC_SUB
-    const int e = last_launch_error();
-    if (e) return e;
-    // advance past the l layers just written
     for (uint32_t j = 0; j < l; j++) {
       in = out;
       out += 4 * count;
       count >>= 1;
     }
-    remaining -= l;
+    layers -= l;
   }
   return 0;
 }
