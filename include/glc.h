@@ -234,7 +234,7 @@ glc_status glc_commit_batch_fused_cancellable(const glc_commit_job *jobs, uint32
  * Released with glc_mapped_word_destroy(host). */
 glc_status glc_mapped_word_create(uint32_t **host, uint32_t **device);
 glc_status glc_mapped_word_destroy(uint32_t *host);
-/* Waits of glc_commit_batch_fused, and of NTT kernels for the tensor cores, that expired on the
+/* Waits of glc_commit_batch_fused, and of NTT and hash kernels for the tensor cores, that expired on the
  * current device since the library was loaded (0 unless something is wrong; a launch with an expired
  * wait computes wrong results).
  * Synchronous. */

@@ -608,8 +608,10 @@ extern "C" glc_status glc_commit_batch_fused_timeouts(uint64_t *out) {
   unsigned long long v = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&v, g_fused_timeouts, sizeof(v));
   uint64_t ntt = 0;
+  unsigned long long p2 = 0;
   if (e == cudaSuccess) e = (cudaError_t)ntt_expired_waits(&ntt);
-  v += ntt;
+  if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&p2, tc::d_p2_expired, sizeof(p2));
+  v += ntt + p2;
   *out = v;
   return (int)e;
 }

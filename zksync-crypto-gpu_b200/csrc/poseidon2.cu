@@ -9,10 +9,13 @@
 //    the next round's constants are added before that reduction, so a round constant costs no
 //    modular addition;
 //  * round constants live in __constant__ memory (uniform across a warp: one broadcast read);
+//  * launches that fill it several times over run the partial rounds on the tensor cores
+//    (p2_tensor.cuh);
 //  * launches that cannot fill the GPU with one thread per permutation take four lanes per
 //    permutation (p2_spread.cuh), and a tree's narrow layers run as fused subtrees, up to 7 layers a
 //    launch.
 #include <algorithm>
+#include <atomic>
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
@@ -38,11 +41,16 @@ struct ExternalConstants {
   double rcd[32][WIDTH][2];
 };
 static constexpr double TWO52 = 4503599627370496.0;
+// (0x433 << 52) (1 + 2^32) mod p: the exponent bits of the two halves as fold() sums them.  The
+// constants are stored minus this, so the bits are not masked off.
+static constexpr uint64_t EXPONENT_BITS =
+    (uint64_t)((((unsigned __int128)0x433 << 52) + ((unsigned __int128)0x433 << 84)) % P);
 constexpr ExternalConstants make_external_constants(const uint64_t (&rc)[ROUNDS][WIDTH]) {
   ExternalConstants t{};
   for (uint32_t r = 0; r < 32; r++)
     for (uint32_t i = 0; i < WIDTH; i++) {
-      const uint64_t v = r < ROUNDS ? rc[r][i] : (r == RC_ROW_PARTIAL_ENTRY && i == 0 ? rc[4][0] : 0);
+      const uint64_t c = (r < ROUNDS ? rc[r][i] : (r == RC_ROW_PARTIAL_ENTRY && i == 0 ? rc[4][0] : 0)) % P;
+      const uint64_t v = c >= EXPONENT_BITS ? c - EXPONENT_BITS : c + (P - EXPONENT_BITS);
       t.rcd[r][i][0] = TWO52 + (double)(uint32_t)v;
       t.rcd[r][i][1] = TWO52 + (double)(uint32_t)(v >> 32);
     }
@@ -65,8 +73,9 @@ __device__ __forceinline__ uint64_t sbox(uint64_t x) {
 // and multiply-adds by 2 and 4 are exact: the layer runs on the otherwise idle FP64 pipe while
 // the integer pipes carry the S-box products.  The results come back through the exponent
 // trick: for an integer 0 <= x < 2^52, the bits of x + 2^52 are 0x433 << 52 | x, and the
-// addend 2^52 + (half of the next round's constant) adds that constant for free.  fold() then
-// combines the two halves into one 64-bit value.  Measured on B200: 2.4% faster per
+// addend 2^52 + (half of the next round's constant) adds that constant for free; the exponent bits
+// stay in and the constants make up for them.  fold() then combines the two halves into one 64-bit
+// value (its bound holds: the exponent bits sum to 2^63.07).  Measured on B200: 2.4% faster per
 // permutation than the same layer in 64-bit integer adds.
 
 // M4 of eprint 2023/323 Appendix B (poseidon2_gl.cuh:11-25)
@@ -80,7 +89,21 @@ __device__ __forceinline__ void m4(double &x0, double &x1, double &x2, double &x
   x3 = t4;
 }
 
+// fold() with one multiply-add instead of two, for code whose busiest pipe is the multipliers': the
+// sum of A and hi32(B) * EPS + lo32(B) * 2^32 by carry chains, then EPS times its top word.
+__device__ __forceinline__ uint64_t fold_alu(uint64_t A, uint64_t B) {
+  uint32_t r0, r1, k;
+  asm("{\n\t.reg .u32 u;\n\t"
+      "sub.cc.u32 %0, %3, %6;\n\tsubc.u32 u, %6, 0;\n\t"
+      "add.cc.u32 %1, %4, u;\n\taddc.u32 %2, 0, 0;\n\t"
+      "add.cc.u32 %1, %1, %5;\n\taddc.u32 %2, %2, 0;\n\t}"
+      : "=&r"(r0), "=&r"(r1), "=&r"(k)
+      : "r"(lo32(A)), "r"(hi32(A)), "r"(lo32(B)), "r"(hi32(B)));
+  return madw(k, 0xFFFFFFFFu, pack(r0, r1));
+}
+
 // s <- M_E s + the constants of row `row` of c_ext
+template <bool ALU_FOLD = false>
 __device__ __forceinline__ void external_layer(uint64_t s[WIDTH], uint32_t row) {
   double xl[WIDTH], xh[WIDTH];
 #pragma unroll
@@ -107,9 +130,9 @@ __device__ __forceinline__ void external_layer(uint64_t s[WIDTH], uint32_t row) 
   const double(*rcd)[2] = c_ext.rcd[row];
 #pragma unroll
   for (int i = 0; i < WIDTH; i++) {
-    const uint64_t A = (uint64_t)__double_as_longlong(L[i] + rcd[i][0]) & 0x000FFFFFFFFFFFFFull;
-    const uint64_t B = (uint64_t)__double_as_longlong(H[i] + rcd[i][1]) & 0x000FFFFFFFFFFFFFull;
-    s[i] = fold(A, B);
+    const uint64_t A = (uint64_t)__double_as_longlong(L[i] + rcd[i][0]);
+    const uint64_t B = (uint64_t)__double_as_longlong(H[i] + rcd[i][1]);
+    s[i] = ALU_FOLD ? fold_alu(A, B) : fold(A, B);
   }
 }
 
@@ -299,6 +322,7 @@ __device__ __forceinline__ void permutation(uint64_t s[WIDTH]) {
 
 }  // namespace glc
 #include "p2_spread.cuh"
+#include "p2_tensor.cuh"
 namespace glc {
 
 // Leaf hashes (poseidon2_gl_st.cu:25-59): leaf i absorbs values[(i<<r) + row + col*rows*count]
@@ -308,14 +332,15 @@ namespace glc {
 // (three 256-thread CTAs), MINB = 5 allows 102 with at most 128 threads per CTA (five CTAs).
 __host__ __device__ constexpr int leaf_max_threads(int minb) { return minb == 5 ? 128 : 256; }
 // The leaf hash of leaf gid (one thread's work in p2_leaves_kernel and in the fused batch kernel).
-template <int ROLL, bool LAZY>
-__device__ __forceinline__ void leaf_hash(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint64_t cols,
-                                          uint64_t count, bool load_intermediate, bool store_intermediate,
-                                          uint64_t gid) {
+// permute(s) replaces the state; a thread that is not `live` only takes part in it.
+template <class Permute>
+__device__ __forceinline__ void leaf_absorb(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint64_t cols,
+                                            uint64_t count, bool load_intermediate, bool store_intermediate,
+                                            uint64_t gid, bool live, Permute &&permute) {
   uint64_t s[WIDTH];
 #pragma unroll
   for (int i = 0; i < WIDTH; i++) s[i] = 0;
-  if (load_intermediate) {
+  if (load_intermediate && live) {
 #pragma unroll
     for (int k = 0; k < 4; k++) s[8 + k] = results[gid + k * count];
   }
@@ -329,7 +354,7 @@ __device__ __forceinline__ void leaf_hash(const uint64_t *values, uint64_t *resu
   uint64_t nxt[8];
 #pragma unroll
   for (int i = 0; i < 8; i++)
-    nxt[i] = (uint64_t)i < total ? __ldcs(v + ((uint64_t)i & (rows - 1)) + ((uint64_t)i >> log_rows) * col_stride) : 0;
+    nxt[i] = live && (uint64_t)i < total ? __ldcs(v + ((uint64_t)i & (rows - 1)) + ((uint64_t)i >> log_rows) * col_stride) : 0;
   for (uint64_t off = 0; off < total; off += 8) {
 #pragma unroll
     for (int i = 0; i < 8; i++) s[i] = nxt[i];
@@ -337,13 +362,21 @@ __device__ __forceinline__ void leaf_hash(const uint64_t *values, uint64_t *resu
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const uint64_t o = off + 8 + i;
-        nxt[i] = o < total ? __ldcs(v + (o & (rows - 1)) + (o >> log_rows) * col_stride) : 0;
+        nxt[i] = live && o < total ? __ldcs(v + (o & (rows - 1)) + (o >> log_rows) * col_stride) : 0;
       }
     }
-    permutation<ROLL, LAZY>(s);
+    permute(s);
   }
+  if (!live) return;
 #pragma unroll
   for (int k = 0; k < 4; k++) results[gid + k * count] = canon(store_intermediate ? s[8 + k] : s[k]);
+}
+template <int ROLL, bool LAZY>
+__device__ __forceinline__ void leaf_hash(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint64_t cols,
+                                          uint64_t count, bool load_intermediate, bool store_intermediate,
+                                          uint64_t gid) {
+  leaf_absorb(values, results, log_rows, cols, count, load_intermediate, store_intermediate, gid, true,
+              [](uint64_t(&s)[WIDTH]) { permutation<ROLL, LAZY>(s); });
 }
 
 template <int ROLL, bool LAZY, int MINB>
@@ -353,6 +386,41 @@ __global__ void __launch_bounds__(leaf_max_threads(MINB), MINB) p2_leaves_kernel
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= count) return;
   leaf_hash<ROLL, LAZY>(values, results, log_rows, cols, count, load_intermediate, store_intermediate, gid);
+}
+
+// Leaves and nodes with the partial rounds on the tensor cores: a CTA of five warpgroups, each
+// hashing tiles of 128 leaves or nodes.  Tile s of the launch goes to CTA s % gridDim.x, so a
+// launch of few tiles spreads them over the SMs.
+__global__ void __launch_bounds__(tc::TILE *tc::GROUPS, 1)
+    p2_leaves_tensor_kernel(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint32_t total, uint64_t count,
+                            bool load_intermediate, bool store_intermediate) {
+  tc::Group g = tc::setup();
+  const uint32_t tiles = (uint32_t)((count + tc::TILE - 1) / tc::TILE);
+  // value o of leaf i: row o % rows of column o / rows
+  auto load = [&](uint32_t tile, uint32_t o) -> uint64_t {
+    const uint64_t i = (uint64_t)tile * tc::TILE + tc::thread() % tc::TILE;
+    const uint32_t rows = 1u << log_rows;
+    return i < count && o < total ? __ldcs(values + ((((uint64_t)(o >> log_rows) * count + i) << log_rows) + (o & (rows - 1)))) : 0;
+  };
+  for (uint32_t t = tc::Group::index() * gridDim.x + blockIdx.x; t < tiles; t += tc::GROUPS * gridDim.x) {
+    uint64_t s[WIDTH];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint64_t i = (uint64_t)t * tc::TILE + threadIdx.x % tc::TILE;
+      s[8 + k] = load_intermediate && i < count ? results[i + k * count] : 0;
+    }
+    for (uint32_t off = 0; off < total; off += 8) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) s[k] = load(t, off + k);
+      tc::permutation(s, g);
+    }
+    const uint64_t i = (uint64_t)t * tc::TILE + threadIdx.x % tc::TILE;
+    if (i < count) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) results[i + k * count] = store_intermediate ? s[8 + k] : s[k];
+    }
+  }
+  tc::teardown();
 }
 
 // Node hashes (poseidon2_gl_st.cu:61-82): node i = P2(L0..L3, R0..R3, 0,0,0,0)[0..4] with
@@ -398,6 +466,29 @@ __global__ void __launch_bounds__(256) p2_nodes_kernel(const uint64_t *values, u
   hash_node<ROLL, LAZY>(l, r, o);
 #pragma unroll
   for (int k = 0; k < 4; k++) results[k * count + gid] = o[k];
+}
+
+__global__ void __launch_bounds__(tc::TILE *tc::GROUPS, 1)
+    p2_nodes_tensor_kernel(const uint64_t *values, uint64_t *results, uint64_t count, bool aligned) {
+  tc::Group g = tc::setup();
+  const uint64_t tiles = (count + tc::TILE - 1) / tc::TILE;
+  for (uint64_t t = (uint64_t)(threadIdx.x / tc::TILE) * gridDim.x + blockIdx.x; t < tiles; t += tc::GROUPS * gridDim.x) {
+    const uint64_t gid = t * tc::TILE + threadIdx.x % tc::TILE;
+    uint64_t l[4] = {}, r[4] = {}, s[WIDTH];
+    if (gid < count) load_children(values, count, gid, l, r, aligned);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s[k] = l[k];
+      s[4 + k] = r[k];
+      s[8 + k] = 0;
+    }
+    tc::permutation(s, g);
+    if (gid < count) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) results[k * count + gid] = s[k];
+    }
+  }
+  tc::teardown();
 }
 
 // gather_rows (queries.cuh:9-19)
@@ -470,6 +561,29 @@ static void leaves_go(uint32_t minb, uint32_t blocks, uint32_t threads, cudaStre
 // 16384: 50 / 25.8 / 21.7.
 static constexpr uint64_t HEX_MAX = 2048, QUAD_MAX = 8192;
 
+// From this many leaves or nodes on, a launch runs its partial rounds on the tensor cores (p2_tensor.cuh),
+// unless it shares the GPU with other jobs' small kernels, which its CTAs, one to an SM, would keep
+// out.  Measured on B200, G permutations/s, tensor / a thread each: nodes 2^16 1.25 / 1.20, 2^17 1.50 /
+// 1.49, 2^18 1.67 / 1.56, 2^22 1.77 / 1.66; leaves of 32 columns 2^16 1.42 / 1.35, 2^17 1.59 / 1.58,
+// 2^18 1.71 / 1.62; of 176 columns 2^15 1.16 / 1.28, 2^22 1.75 / 1.69.
+static constexpr uint64_t TENSOR_MIN = 1 << 18;
+
+// One CTA per SM hashes it all: with CTAs of two tiles a group instead, a CTA's last group and the next
+// one's prologue leave the SM half idle (2^21 leaves of 128 columns: 1.63 G permutations/s, 1.74 so).
+static uint32_t tensor_grid(uint64_t count) { return (uint32_t)std::min<uint64_t>((count + tc::TILE - 1) / tc::TILE, 148); }
+static cudaError_t tensor_attributes() {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  static std::atomic<bool> done[MAX_DEVICES];
+  if (dev < MAX_DEVICES && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  e = cudaFuncSetAttribute(p2_leaves_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(p2_nodes_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
+  if (e == cudaSuccess && dev < MAX_DEVICES) done[dev].store(true, std::memory_order_release);
+  return e;
+}
+
 static uint32_t spread_grid(uint64_t count, uint32_t lanes) {
   return (uint32_t)((count * lanes + SPREAD_THREADS - 1) / SPREAD_THREADS);
 }
@@ -485,6 +599,13 @@ int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_row
     else
       p2_leaves_spread_kernel<4><<<spread_grid(count, 4), SPREAD_THREADS, 0, stream>>>(
           values, results, log_rows, cols, count, load_intermediate, store_intermediate);
+    return last_launch_error();
+  }
+  if (count >= TENSOR_MIN && together != ~0ull && cols && (cols << log_rows) <= 0xfffffff0u) {
+    const cudaError_t e = tensor_attributes();
+    if (e != cudaSuccess) return (int)e;
+    p2_leaves_tensor_kernel<<<tensor_grid(count), tc::TILE * tc::GROUPS, tc::SMEM_BYTES, stream>>>(
+        values, results, log_rows, (uint32_t)(cols << log_rows), count, load_intermediate, store_intermediate);
     return last_launch_error();
   }
   const P2Tuning &tu = p2_tuning();
@@ -518,6 +639,13 @@ int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, c
   const uint64_t blocks = (count + threads - 1) / threads;
   if (blocks > 0x7fffffffull) return fail("poseidon2: too many nodes");
   const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15) == 0;
+  if (count >= TENSOR_MIN) {
+    const cudaError_t e = tensor_attributes();
+    if (e != cudaSuccess) return (int)e;
+    p2_nodes_tensor_kernel<<<tensor_grid(count), tc::TILE * tc::GROUPS, tc::SMEM_BYTES, stream>>>(values, results,
+                                                                                                  count, aligned);
+    return last_launch_error();
+  }
 #define GLC_NODES(R, L) p2_nodes_kernel<R, L><<<(uint32_t)blocks, threads, 0, stream>>>(values, results, count, aligned)
   GLC_P2_VARIANT(tu, GLC_NODES);
 #undef GLC_NODES
@@ -556,6 +684,13 @@ int p2_install_round_constants(const uint64_t *rc) {
     static ExternalConstants ext;  // large; built on the host, copied once
     ext = make_external_constants(t);
     e = cudaMemcpyToSymbol(c_ext, &ext, sizeof(ext));
+  }
+  if (e == cudaSuccess) {
+    uint64_t t[ROUNDS][WIDTH];
+    for (uint32_t r = 0; r < ROUNDS; r++)
+      for (uint32_t i = 0; i < WIDTH; i++) t[r][i] = rc[r * WIDTH + i];
+    const tc::Matrices m = tc::make_matrices(t);
+    e = cudaMemcpyToSymbol(tc::d_matrices, &m, sizeof(m));
   }
   if (e == cudaSuccess && dev >= 0 && dev < MAX_DEVICES) g_rc_installed[dev] = true;
   return (int)e;
