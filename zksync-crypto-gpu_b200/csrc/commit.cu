@@ -16,6 +16,7 @@
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
+#include "launch.cuh"
 
 namespace glc {
 
@@ -24,6 +25,7 @@ __global__ void gather_caps_kernel(const uint64_t *trees, uint64_t tree_len, uin
                                    uint32_t cosets, uint64_t *cap) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t total = 4 * ccap * cosets;
+  dependency_wait();
   if (t >= total) return;
   const uint32_t m = t % ccap, c = (t / ccap) % cosets, j = t / (ccap * cosets);
   cap[(uint64_t)j * ccap * cosets + (uint64_t)c * ccap + m] = trees[c * tree_len + cap_off + (uint64_t)j * ccap + m];
@@ -140,7 +142,7 @@ int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *ev
   cur = stream;
   const uint32_t ccap = 1u << log_ccap;
   const uint32_t total = 4 * ccap * f;
-  gather_caps_kernel<<<(total + 127) / 128, 128, 0, stream>>>(j.trees, 8 * n, 8 * n - 8ull * ccap, ccap, f, j.cap);
+  launch(gather_caps_kernel, dim3((total + 127) / 128), 128, 0, stream, j.trees, 8 * n, 8 * n - 8ull * ccap, ccap, f, j.cap);
   e = last_launch_error();
   if (!e) e = mark();
   return e;

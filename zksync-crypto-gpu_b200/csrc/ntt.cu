@@ -26,6 +26,7 @@
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
+#include "launch.cuh"
 #include "ntt_tensor.cuh"
 #include "ntt_tile.cuh"
 
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(pass_threads(RB), pass_min_blocks(RB)) ntt_pas
 __global__ void bitrev_naive_kernel(const uint64_t *src, uint64_t src_stride, uint64_t *dst, uint64_t dst_stride,
                                     uint32_t log_rows) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  dependency_wait();
   if (i >= (1u << log_rows)) return;
   const uint32_t r = log_rows ? __brev(i) >> (32 - log_rows) : 0;
   if (i > r) return;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(256) bitrev_tiled_kernel(const uint64_t *src, 
   const uint32_t hb = h - 5;
   const uint32_t A = blockIdx.x >> hb, B = blockIdx.x & ((1u << hb) - 1);
   const uint32_t As = hb ? __brev(B) >> (32 - hb) : 0, Bs = hb ? __brev(A) >> (32 - hb) : 0;
+  dependency_wait();
   if (A > As || (A == As && B > Bs)) return;  // the image tile's CTA moves this pair
   const uint32_t m = blockIdx.z;
   const uint64_t col = blockIdx.y;
@@ -131,13 +134,13 @@ int bitrev_launch(const uint64_t *src, uint64_t src_stride, uint64_t *dst, uint6
   if (log_rows < 10) {
     const uint32_t n = 1u << log_rows;
     const uint32_t threads = std::min<uint32_t>(n, 256);
-    bitrev_naive_kernel<<<dim3((n + threads - 1) / threads, cols), threads, 0, stream>>>(src, src_stride, dst, dst_stride,
-                                                                                          log_rows);
+    launch(bitrev_naive_kernel, dim3((n + threads - 1) / threads, cols), threads, 0, stream, src, src_stride, dst, dst_stride,
+           log_rows);
   } else {
     const uint32_t h = log_rows >> 1;
     const uint32_t tiles = 1u << (2 * (h - 5));
-    bitrev_tiled_kernel<<<dim3(tiles, cols, 1u << (log_rows & 1)), 256, 0, stream>>>(src, src_stride, dst, dst_stride,
-                                                                                   log_rows);
+    launch(bitrev_tiled_kernel, dim3(tiles, cols, 1u << (log_rows & 1)), 256, 0, stream, src, src_stride, dst, dst_stride,
+           log_rows);
   }
   return last_launch_error();
 }
@@ -217,11 +220,11 @@ int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_n
         b.num_cols = std::min<uint32_t>(cols - y0 * cpc, ycount * cpc);
         const dim3 grid((uint32_t)tiles_per_col, ycount);
         if (tu.radix_bits == 2)
-          ntt_pass_kernel<2><<<grid, threads, smem, stream>>>(b);
+          launch(ntt_pass_kernel<2>, grid, threads, smem, stream, b);
         else if (tu.radix_bits == 4)
-          ntt_pass_kernel<4><<<grid, threads, smem, stream>>>(b);
+          launch(ntt_pass_kernel<4>, grid, threads, smem, stream, b);
         else
-          ntt_pass_kernel<3><<<grid, threads, smem, stream>>>(b);
+          launch(ntt_pass_kernel<3>, grid, threads, smem, stream, b);
       }
       const int e = last_launch_error();
       if (e) return e;

@@ -7,6 +7,7 @@
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
+#include "launch.cuh"
 
 namespace glc {
 
@@ -174,6 +175,7 @@ __device__ __forceinline__ void ntt_pass_tile(const PassArgs &a, uint32_t bx, ui
     for (uint32_t w = threadIdx.x; w < nq; w += blockDim.x)
       Qt[w] = coset_power(a, a.j_bitrev ? brev_low(hi, a.log_n - k) : lo0 + w);
   }
+  dependency_wait();  // the tables above are the context's
   const uint32_t col0 = by * a.cols_per_cta;
   const uint32_t col1 = min(col0 + a.cols_per_cta, a.num_cols);
   const uint32_t wmask = (1u << log_w) - 1;

@@ -19,6 +19,7 @@
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
+#include "launch.cuh"
 
 namespace glc {
 
@@ -497,6 +498,7 @@ __global__ void p2_gather_rows_kernel(const uint32_t *indexes, uint32_t indexes_
                                       uint64_t results_stride, uint64_t cols) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t rows_out = (uint64_t)indexes_count << log_rows_per_index;
+  dependency_wait();
   if (t >= rows_out) return;
   const uint64_t idx = t >> log_rows_per_index, x = t & ((1ull << log_rows_per_index) - 1);
   const uint64_t src_row = ((uint64_t)indexes[idx] << log_rows_per_index) + x;
@@ -508,6 +510,7 @@ __global__ void p2_gather_rows_kernel(const uint32_t *indexes, uint32_t indexes_
 __global__ void p2_gather_paths_kernel(const uint32_t *indexes, uint32_t indexes_count, const uint64_t *values,
                                        uint32_t log_leaves, uint64_t *results, uint32_t layers) {
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+  dependency_wait();
   if (idx >= indexes_count) return;
   const uint32_t col = blockIdx.y, layer = blockIdx.z;
   if (layer >= layers) return;
@@ -817,8 +820,8 @@ extern "C" glc_status glc_poseidon2_gather_rows(const uint32_t *indexes, size_t 
   const uint32_t threads = 128;
   const uint64_t blocks = (results_rows + threads - 1) / threads;
   const uint32_t gy = (uint32_t)std::min<uint64_t>(values_cols, 65535);
-  p2_gather_rows_kernel<<<dim3((uint32_t)blocks, gy), threads, 0, (cudaStream_t)stream>>>(
-      indexes, (uint32_t)indexes_len, log_rows_per_index, values, values_stride, results, results_stride, values_cols);
+  launch(p2_gather_rows_kernel, dim3((uint32_t)blocks, gy), threads, 0, (cudaStream_t)stream,
+         indexes, (uint32_t)indexes_len, log_rows_per_index, values, values_stride, results, results_stride, values_cols);
   return last_launch_error();
 }
 
@@ -839,8 +842,8 @@ extern "C" glc_status glc_poseidon2_gather_merkle_paths(const uint32_t *indexes,
   if (indexes_len == 0 || layers_count == 0) return 0;
   const uint32_t threads = 32;
   const uint32_t blocks = (uint32_t)((indexes_len + threads - 1) / threads);
-  p2_gather_paths_kernel<<<dim3(blocks, 4, layers_count), threads, 0, (cudaStream_t)stream>>>(
-      indexes, (uint32_t)indexes_len, values, log_leaves, results, layers_count);
+  launch(p2_gather_paths_kernel, dim3(blocks, 4, layers_count), threads, 0, (cudaStream_t)stream,
+         indexes, (uint32_t)indexes_len, values, log_leaves, results, layers_count);
   return last_launch_error();
 }
 
