@@ -100,4 +100,6 @@ def check(status: int, where: str) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(lib(), name)(*args), name)
+    status = getattr(_lib or lib(), name)(*args)
+    if status:
+        check(status, name)
