@@ -522,7 +522,7 @@ def run_ours(args, rank, world, local_rank):
                                     frac=max(u["bytes"] / (peaks["hbm_gbs"] * 1e9), u["modmul"] / mm_peak) * 1e3
                                     / max(1e-9, stage[k]))
                             for k, u in stage_units(shape).items()},
-        "roofline": {"bound": "int", "kernel": "p2_leaves_kernel", "achieved": achieved,
+        "roofline": {"bound": "int", "kernel": "p2_leaves_tensor_kernel", "achieved": achieved,
                      "peak": mm_peak / 1e9, "unit": "Gmodmul/s", "frac": achieved * 1e9 / mm_peak,
                      "launch_ms_in_step": leaf_ms, "launch_ms_alone": alone,
                      "frac_alone": leaf_modmul / (alone / 1e3) / mm_peak,
