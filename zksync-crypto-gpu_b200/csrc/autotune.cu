@@ -126,7 +126,7 @@ extern "C" glc_status glc_autotune(uint32_t log_n_min, uint32_t log_n_max, uint3
             ntt_tuning(log_n) = c;
             // time a forward coset LDE (the commitment's dominant NTT), in place
             const float ms = time_ms(s, (int)reps, [&] {
-              return ntt_launch(buf, buf, log_n, nc, 1ull << log_n, 1ull << log_n, false, false, 1, 1, s, 0);
+              return ntt_launch(buf, buf, log_n, nc, 1ull << log_n, 1ull << log_n, false, false, 1, 1, s, 0, true);
             }, &err);
             if (err) break;
             if (ms < best_ms) {
@@ -154,7 +154,7 @@ extern "C" glc_status glc_autotune(uint32_t log_n_min, uint32_t log_n_max, uint3
         c.min_blocks = minb;
         p2_tuning() = c;
         const float ms = time_ms(s, (int)reps, [&] {
-          return p2_leaves_launch(buf, buf + LEAF_COLS * count, 0, LEAF_COLS, count, false, false, s);
+          return p2_leaves_launch(buf, buf + LEAF_COLS * count, 0, LEAF_COLS, count, false, false, s, ~0ull);
         }, &err);
         if (err) break;
         if (ms < best_ms) {

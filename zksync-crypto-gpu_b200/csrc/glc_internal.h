@@ -75,9 +75,10 @@ int p2_install_round_constants(const uint64_t *rc);
 bool p2_constants_installed();
 
 // Internal launchers reused by the commitment pipeline (all enqueue on `stream`).
+// registers_only: the passes that the tuning applies to, however large the batch (for the autotuner).
 int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_ntts, uint64_t in_stride,
                uint64_t out_stride, bool bitrev_inputs, bool inverse, uint32_t log_ext, uint32_t coset_idx,
-               cudaStream_t stream, uint32_t l2_chunk_cols);
+               cudaStream_t stream, uint32_t l2_chunk_cols, bool registers_only = false);
 int bitrev_launch(const uint64_t *src, uint64_t src_stride, uint64_t *dst, uint64_t dst_stride, uint32_t log_rows,
                   uint32_t cols, cudaStream_t stream);
 // together: leaves that other streams hash at the same time, these included (a launch that shares the

@@ -171,14 +171,14 @@ static bool tt_usable(uint32_t log_n, uint32_t num_ntts, bool bitrev_inputs, boo
 
 int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_ntts, uint64_t in_stride,
                uint64_t out_stride, bool bitrev_inputs, bool inverse, uint32_t log_ext, uint32_t coset_idx,
-               cudaStream_t stream, uint32_t l2_chunk_cols) {
+               cudaStream_t stream, uint32_t l2_chunk_cols, bool registers_only) {
   const DeviceTables *t = current_tables();
   if (!t) return fail("NTT: glc_context_create has not been called on this device");
   if (num_ntts == 0) return 0;
   const NttTuning &tu = ntt_tuning(log_n);
   Pass passes[2];
   const uint32_t np = make_plan(log_n, bitrev_inputs, tu, passes);
-  if (tt_usable(log_n, num_ntts, bitrev_inputs, inverse, log_ext)) {
+  if (!registers_only && tt_usable(log_n, num_ntts, bitrev_inputs, inverse, log_ext)) {
     const uint32_t k0 = log_n - TT_LOG;  // strided stages, then 12 contiguous ones
     if (k0 == 0)
       return tt_launch_pass(t, 0, TT_LOG, true, true, in, out, in_stride, out_stride, num_ntts, log_n, bitrev_inputs,
