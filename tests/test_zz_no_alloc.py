@@ -76,3 +76,42 @@ def test_noalloc_limit(glc):
     st = lib.glc_commit_cap_noalloc(ev.data_ptr(), 1 << 20, 20, 120, 1, 4, cap.data_ptr(), None)
     assert st != 0
     assert b"maximum" in lib.glc_last_error_message()
+
+
+RESET = r"""
+import ctypes as C, sys
+L, cu = C.CDLL(sys.argv[1]), C.CDLL("libcuda.so.1")
+log_n, cols = int(sys.argv[2]), int(sys.argv[3])
+L.glc_commit_cap_noalloc.argtypes = [C.c_void_p, C.c_uint64] + 4 * [C.c_uint32] + 2 * [C.c_void_p]
+
+def ok(status, what):
+    assert status == 0, (what, status)
+
+def cap():
+    ok(L.glc_context_create(15, 15), "create")
+    ev, out, host = C.c_uint64(), C.c_uint64(), (C.c_uint64 * 64)()
+    ok(cu.cuMemAlloc_v2(C.byref(ev), C.c_size_t(8 * cols << log_n)), "alloc")
+    ok(cu.cuMemAlloc_v2(C.byref(out), C.c_size_t(512)), "alloc")
+    ok(cu.cuMemsetD32_v2(ev, C.c_uint32(0x12345), C.c_size_t(2 * cols << log_n)), "set")
+    ok(L.glc_commit_cap_noalloc(ev.value, 1 << log_n, log_n, cols, 0, 4, out.value, None), "commit")
+    ok(cu.cuCtxSynchronize(), "synchronize")
+    ok(cu.cuMemcpyDtoH_v2(host, out, C.c_size_t(512)), "copy")
+    ok(L.glc_context_destroy(), "destroy")
+    return list(host)
+
+first = cap()
+ok(cu.cuDevicePrimaryCtxReset_v2(0), "reset")
+assert cap() == first
+print("same")
+"""
+
+
+@pytest.mark.parametrize("log_n,cols", [(12, 8), (16, 100), (19, 8)])
+def test_cap_after_a_device_reset(glc, log_n, cols):
+    """glc_context_destroy, a device reset and glc_context_create may come between two calls, whatever
+    kernels the size takes.  In a process of its own: the reset ends the context."""
+    import subprocess
+    import sys
+    p = subprocess.run([sys.executable, "-c", RESET, glc.LIB_PATH, str(log_n), str(cols)], capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0 and "same" in p.stdout, p.stdout + p.stderr

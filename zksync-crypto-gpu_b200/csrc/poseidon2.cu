@@ -15,7 +15,6 @@
 //    permutation (p2_spread.cuh), and a tree's narrow layers run as fused subtrees, up to 7 layers a
 //    launch.
 #include <algorithm>
-#include <atomic>
 
 #include "glc_field.cuh"
 #include "glc_internal.h"
@@ -574,17 +573,15 @@ static constexpr uint64_t TENSOR_MIN = 1 << 18;
 // One CTA per SM hashes it all: with CTAs of two tiles a group instead, a CTA's last group and the next
 // one's prologue leave the SM half idle (2^21 leaves of 128 columns: 1.63 G permutations/s, 1.74 so).
 static uint32_t tensor_grid(uint64_t count) { return (uint32_t)std::min<uint64_t>((count + tc::TILE - 1) / tc::TILE, 148); }
-static cudaError_t tensor_attributes() {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  static std::atomic<bool> done[MAX_DEVICES];
-  if (dev < MAX_DEVICES && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
-  e = cudaFuncSetAttribute(p2_leaves_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(p2_nodes_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
-  if (e == cudaSuccess && dev < MAX_DEVICES) done[dev].store(true, std::memory_order_release);
-  return e;
+// Launches with the shared memory of the five groups.  The kernel's attribute is set at every launch (a
+// host call of well under a microsecond before 150 us or more of hashing) and not remembered: a device
+// reset takes it along with the context.
+template <typename... Params, typename... Args>
+static int tensor_launch(void (*kernel)(Params...), uint64_t count, cudaStream_t stream, Args... args) {
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
+  if (e != cudaSuccess) return (int)e;
+  kernel<<<tensor_grid(count), tc::TILE * tc::GROUPS, tc::SMEM_BYTES, stream>>>(static_cast<Params>(args)...);
+  return last_launch_error();
 }
 
 static uint32_t spread_grid(uint64_t count, uint32_t lanes) {
@@ -605,11 +602,8 @@ int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_row
     return last_launch_error();
   }
   if (count >= TENSOR_MIN && together != ~0ull && cols && (cols << log_rows) <= 0xfffffff0u) {
-    const cudaError_t e = tensor_attributes();
-    if (e != cudaSuccess) return (int)e;
-    p2_leaves_tensor_kernel<<<tensor_grid(count), tc::TILE * tc::GROUPS, tc::SMEM_BYTES, stream>>>(
-        values, results, log_rows, (uint32_t)(cols << log_rows), count, load_intermediate, store_intermediate);
-    return last_launch_error();
+    return tensor_launch(p2_leaves_tensor_kernel, count, stream, values, results, log_rows, (uint32_t)(cols << log_rows),
+                         count, load_intermediate, store_intermediate);
   }
   const P2Tuning &tu = p2_tuning();
   const uint32_t threads = tu.leaf_threads;
@@ -642,13 +636,7 @@ int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, c
   const uint64_t blocks = (count + threads - 1) / threads;
   if (blocks > 0x7fffffffull) return fail("poseidon2: too many nodes");
   const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15) == 0;
-  if (count >= TENSOR_MIN) {
-    const cudaError_t e = tensor_attributes();
-    if (e != cudaSuccess) return (int)e;
-    p2_nodes_tensor_kernel<<<tensor_grid(count), tc::TILE * tc::GROUPS, tc::SMEM_BYTES, stream>>>(values, results,
-                                                                                                  count, aligned);
-    return last_launch_error();
-  }
+  if (count >= TENSOR_MIN) return tensor_launch(p2_nodes_tensor_kernel, count, stream, values, results, count, aligned);
 #define GLC_NODES(R, L) p2_nodes_kernel<R, L><<<(uint32_t)blocks, threads, 0, stream>>>(values, results, count, aligned)
   GLC_P2_VARIANT(tu, GLC_NODES);
 #undef GLC_NODES
