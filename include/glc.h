@@ -234,10 +234,7 @@ glc_status glc_commit_batch_fused_cancellable(const glc_commit_job *jobs, uint32
  * Released with glc_mapped_word_destroy(host). */
 glc_status glc_mapped_word_create(uint32_t **host, uint32_t **device);
 glc_status glc_mapped_word_destroy(uint32_t *host);
-/* Waits of glc_commit_batch_fused, and of NTT and hash kernels for the tensor cores, that expired on the
- * current device since the library was loaded (0 unless something is wrong; a launch with an expired
- * wait computes wrong results).
- * Synchronous. */
+/* glc_expired_waits under its first name. */
 glc_status glc_commit_batch_fused_timeouts(uint64_t *out);
 
 /* A batch captured once into a CUDA graph and replayed with one launch.  The graph keeps the
@@ -331,6 +328,16 @@ glc_status glc_tuning_load(const char *path);
 /* Elements offset .. offset+count of the seeded synthetic stream: ChaCha20 (RFC 8439) keyed by
  * key32, little-endian u64 words, a word >= p redrawn from the nonce-1 stream (uniform in [0, p)). */
 glc_status glc_fill_random(uint64_t *dst, uint64_t count, uint64_t offset, const uint8_t *key32, void *stream);
+/* Bounded waits that gave up on the current device since the library was loaded, counted by thread: of
+ * glc_batch_ntt_*, glc_poseidon2_* and glc_commit* kernels for the tensor cores, and of
+ * glc_commit_batch_fused for an item's producers.  0 unless something is wrong: such a launch runs to
+ * its end with wrong results.  Launches are asynchronous, so the calls have returned 0 by then; a program
+ * that wants to know reads this after it has synchronised.  glc_server_* does, and fails every request
+ * that the wait may have been part of (cudaErrorTimeout).  Synchronous. */
+glc_status glc_expired_waits(uint64_t *out);
+/* One CTA of 128 threads whose wait for the tensor cores gives up after `polls` (at most 50000) polls of
+ * up to 20 us, counted in glc_expired_waits: for checking that a program notices. */
+glc_status glc_expired_wait_probe(uint32_t polls, void *stream);
 /* Number of kernel launches this library has issued in this process (all devices). */
 uint64_t glc_launch_count(void);
 /* Modular-multiply throughput probe: blocks x 256 threads, 8 independent chains of `iters`

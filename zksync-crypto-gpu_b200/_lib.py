@@ -64,6 +64,8 @@ SIGNATURES = {
     "glc_mapped_word_create": (C.c_int, [vp, vp]),
     "glc_mapped_word_destroy": (C.c_int, [vp]),
     "glc_commit_batch_fused_timeouts": (C.c_int, [vp]),
+    "glc_expired_waits": (C.c_int, [vp]),
+    "glc_expired_wait_probe": (C.c_int, [u32, vp]),
     "glc_commit_graph_create": (C.c_int, [vp, u32, u32, vp]),
     "glc_commit_graph_launch": (C.c_int, [vp, vp]),
     "glc_commit_graph_destroy": (C.c_int, [vp]),

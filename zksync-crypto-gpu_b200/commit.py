@@ -162,7 +162,7 @@ def fused_trace_summary(records) -> dict:
 
 
 def fused_timeouts() -> int:
-    """Expired waits of commit_batch_fused on this device since load (0 unless something is wrong)."""
+    """context.expired_waits() under its first name."""
     v = C.c_uint64()
     call("glc_commit_batch_fused_timeouts", C.byref(v))
     return v.value

@@ -2,9 +2,20 @@
 (crates/boojum-cuda/src/context.rs:157-297)."""
 from __future__ import annotations
 
+import ctypes as C
+
 from ._lib import call
 
 OMEGA_LOG_ORDER = 30
+
+
+def expired_waits() -> int:
+    """Bounded waits of kernels on this device that gave up since load (glc_expired_waits): 0 unless
+    something is wrong.  NTT, hash and commitment calls are asynchronous and cannot report one; results
+    are sound if this did not grow over a synchronisation after them.  Synchronous."""
+    v = C.c_uint64()
+    call("glc_expired_waits", C.byref(v))
+    return v.value
 
 
 class Context:

@@ -117,6 +117,7 @@ extern "C" glc_status glc_context_create(uint32_t powers_of_w_coarse_log_count, 
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = (cudaError_t)ntt_init_device();
   if (e == cudaSuccess) e = (cudaError_t)ntt_dft_create(&t.dft);
+  if (e == cudaSuccess) e = (cudaError_t)expired_counter(&t.expired);
   if (e != cudaSuccess) {
     free_tables(t);
     return (int)e;

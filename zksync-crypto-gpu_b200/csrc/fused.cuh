@@ -74,9 +74,6 @@ struct FusedEntry {
   uint32_t ccap;           // caps: cap entries per coset
 };
 
-// Waits that expired (device-wide, since the library was loaded).
-static __device__ unsigned long long g_fused_timeouts;
-
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -159,7 +156,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 3)
         uint32_t it = 0;
         while (ld_acquire(counters + E.dep) < E.dep_target && !ld_acquire(abort_flag)) {
           if (++it > FUSED_WAIT_LIMIT) {
-            atomicAdd(&g_fused_timeouts, 1ull);
+            atomicAdd(&d_expired, 1ull);
             atomicExch(abort_flag, 1u);
             break;
           }
@@ -605,13 +602,5 @@ extern "C" glc_status glc_mapped_word_destroy(uint32_t *host) { return host ? (i
 
 extern "C" glc_status glc_commit_batch_fused_timeouts(uint64_t *out) {
   if (!out) return fail("commit_batch_fused_timeouts: null output");
-  unsigned long long v = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&v, g_fused_timeouts, sizeof(v));
-  uint64_t ntt = 0;
-  unsigned long long p2 = 0;
-  if (e == cudaSuccess) e = (cudaError_t)ntt_expired_waits(&ntt);
-  if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&p2, tc::d_p2_expired, sizeof(p2));
-  v += ntt + p2;
-  *out = v;
-  return (int)e;
+  return glc_expired_waits(out);
 }

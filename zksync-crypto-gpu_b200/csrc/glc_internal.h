@@ -33,6 +33,7 @@ struct DeviceTables {
   // Byte matrices of the small DFTs of the tensor-core NTT passes (ntt_tensor.cuh): forward n2b,
   // forward b2n, inverse n2b, inverse b2n.
   uint8_t *dft = nullptr;
+  unsigned long long *expired = nullptr;  // the device's count of waits that gave up (glc_expired_waits)
 };
 
 // Tables of the current device, or nullptr when glc_context_create has not run on it.
@@ -91,7 +92,7 @@ int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, c
 int p2_tree_nodes_launch(uint64_t *layer0, uint64_t leaves, uint32_t layers, cudaStream_t stream);
 
 int ntt_init_device();  // kernel attributes; called by glc_context_create
-int ntt_expired_waits(uint64_t *out);  // waits for the tensor cores that gave up on this device
+int expired_counter(unsigned long long **out);  // device address of the count of waits that gave up
 int ntt_dft_create(uint8_t **out);  // the tables' byte matrices; called by glc_context_create
 void noalloc_forget_device(int dev);  // drops the cached scratch address; called by glc_context_destroy
 void fused_forget_device(int dev);    // releases the fused batch's work-table pool; called by glc_context_destroy

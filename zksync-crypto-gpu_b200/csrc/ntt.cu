@@ -99,13 +99,6 @@ int ntt_init_device() {
   return (int)e;
 }
 
-int ntt_expired_waits(uint64_t *out) {
-  unsigned long long v = 0;
-  const cudaError_t e = cudaMemcpyFromSymbol(&v, d_ntt_expired, sizeof(v));
-  *out = v;
-  return (int)e;
-}
-
 int ntt_dft_create(uint8_t **out) {
   std::vector<uint8_t> m(4 * DFT_BYTES);
   for (uint32_t v = 0; v < 4; v++)

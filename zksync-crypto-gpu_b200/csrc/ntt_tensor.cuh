@@ -64,7 +64,8 @@ struct TensorPass {
   uint32_t last;         // canonical output
   uint32_t staged;       // contiguous n2b pass whose output is not 32-byte aligned: a thread's 16
                          // consecutive values go out through shared memory instead of 32-byte stores
-  uint32_t smem_bar;
+  uint32_t smem_bar;     // mbarrier, TMEM address, the barrier of tc::finish: 8 bytes each
+  unsigned long long *expired;  // counts the waits that gave up
   const uint64_t *tw;
   const uint8_t *dft;
   uint64_t scale;        // N^-1 on an inverse's last pass, else 1
@@ -74,8 +75,6 @@ struct TensorPass {
 // Twiddle j of block m of a round with nblk blocks: word j * (nblk + 2) + m of its table (two words
 // of padding a row: a half-warp reading 8 rows hits different banks).
 __host__ __device__ constexpr uint32_t tt_table_words(uint32_t r, uint32_t nblk) { return (nblk + 2) << r; }
-
-__device__ unsigned long long d_ntt_expired;  // waits for the tensor cores that gave up
 
 // g of block m (of the round's first stage) of round q
 __device__ __forceinline__ uint64_t tt_twiddle(const TensorPass &a, uint32_t q, uint64_t m) {
@@ -317,7 +316,7 @@ __global__ void __launch_bounds__(TT_THREADS, 2) ntt_tensor_kernel(const __grid_
         tc::commit(bar);
       }
       __syncwarp();
-      if (!tc::mbar_wait(bar, phase) && threadIdx.x == 0) atomicAdd(&d_ntt_expired, 1ull);
+      tc::mbar_wait(bar, phase, a.expired);
       if (n + 1 < a.rounds) {
         tt_round_any<DIF, false>(a, q, tmem_lanes, smem_a, words, nullptr);
       } else {
@@ -335,12 +334,7 @@ __global__ void __launch_bounds__(TT_THREADS, 2) ntt_tensor_kernel(const __grid_
       }
     }
   }
-  tc::fence_before();
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    tc::fence_after();
-    tc::tmem_free<TT_COLUMNS>(tmem);
-  }
+  tc::finish<TT_COLUMNS>(tmem, phase, bar + 16, (threadIdx.x & 127) == 0, 2, a.expired);
 }
 
 // ---- host side ----
@@ -428,7 +422,8 @@ inline int tt_launch_pass(const DeviceTables *t, uint32_t s0, uint32_t k, bool f
     if (q || a.plain_first) a.radices |= 1u << a.r[q];
   }
   a.smem_bar = words * 8;
-  const size_t smem = (size_t)a.smem_bar + 16;
+  const size_t smem = (size_t)a.smem_bar + 24;
+  a.expired = t->expired;
   a.staged = !bitrev_inputs && a.log_m == 0 && ((reinterpret_cast<uintptr_t>(out) & 31) || (out_stride & 3));
   a.tw = inverse ? t->tw_inv : t->tw_fwd;
   a.dft = t->dft + ((inverse ? 2 : 0) + (bitrev_inputs ? 1 : 0)) * DFT_BYTES;

@@ -47,8 +47,9 @@ __host__ __device__ constexpr uint32_t y_offset(uint32_t b) { return Y_COLS * 16
 static constexpr uint32_t OUT_OFFSET = Y_COLS * 16 * (7 * BLOCKS + BLOCKS * (BLOCKS - 1));
 static constexpr uint32_t ZERO_OFFSET = OUT_OFFSET + OUT_COLS * 16 * CHUNKS;
 static constexpr uint32_t B_BYTES = ZERO_OFFSET + OUT_COLS * 16;
-static constexpr uint32_t SMEM_TAIL = B_BYTES + GROUPS * A_BYTES;  // mbarriers, TMEM address
-static constexpr uint32_t SMEM_BYTES = SMEM_TAIL + 8 * GROUPS + 8;
+static constexpr uint32_t SMEM_TAIL = B_BYTES + GROUPS * A_BYTES;  // mbarriers, TMEM address, finish()'s barrier
+static constexpr uint32_t SMEM_DRAIN = SMEM_TAIL + 8 * GROUPS + 8;
+static constexpr uint32_t SMEM_BYTES = SMEM_DRAIN + 8;
 
 struct Matrices {
   alignas(16) uint8_t b[B_BYTES];
@@ -142,8 +143,6 @@ static constexpr Matrices k_matrices = make_matrices(k_placeholder_rc);
 static_assert(digits_fit(k_matrices), "a digit sum is too large");
 __device__ Matrices d_matrices = k_matrices;
 
-__device__ unsigned long long d_p2_expired;  // waits for the tensor cores that gave up
-
 // One warpgroup's share of the CTA's tensor-core resources.  Only the phase is kept; the addresses
 // are cheap to compute again (thread() keeps the compiler from holding them in registers, which the
 // full rounds need).
@@ -165,20 +164,19 @@ struct Group {
     return smem_addr(smem) + B_BYTES + (t / TILE) * A_BYTES + (t % TILE) * 16;
   }
   __device__ __forceinline__ static uint32_t bar() { return smem_addr(smem) + SMEM_TAIL + 8 * index(); }
-  // first TMEM column of the group, at lane 0 (where the products go); the CTA holds all 512
-  __device__ __forceinline__ static uint32_t tmem() {
+  // the CTA's TMEM, all 512 columns, and the first column of the group, at lane 0 (where the products go)
+  __device__ __forceinline__ static uint32_t base() {
     uint32_t base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(base) : "r"(smem_addr(smem) + SMEM_TAIL + 8 * GROUPS) : "memory");
-    return base + index() * OUT_COLS;
+    return base;
   }
+  __device__ __forceinline__ static uint32_t tmem() { return base() + index() * OUT_COLS; }
   // the same column at this warp's quarter of the lanes (what it may read)
   __device__ __forceinline__ static uint32_t lanes() { return tmem() + ((thread() % TILE & ~31u) << 16); }
 };
 
 // Every thread of the group waits until the products issued so far are done.
-__device__ __forceinline__ void wait(Group &g) {
-  if (!mbar_wait(g.bar(), g.phase) && g.leader()) atomicAdd(&d_p2_expired, 1ull);
-}
+__device__ __forceinline__ void wait(Group &g) { mbar_wait(g.bar(), g.phase, &d_expired); }
 
 // Makes the group's shared-memory rows visible to the tensor cores and orders its TMEM reads
 // before the products issued next.
@@ -294,13 +292,29 @@ __device__ __forceinline__ Group setup() {
   fence_after();
   return {0};
 }
-__device__ __forceinline__ void teardown() {
+__device__ __forceinline__ void teardown(const Group &g) {
+  finish<512>(Group::base(), g.phase, smem_addr(smem) + SMEM_DRAIN, Group::leader(), GROUPS, &d_expired);
+}
+
+// One CTA whose wait runs out: a product is issued, and nothing completes the barrier waited on.
+__global__ void __launch_bounds__(TILE) expired_wait_kernel(uint32_t polls) {
+  __shared__ __align__(128) uint8_t rows[TILE * 32 + Y_COLS * 32];
+  __shared__ __align__(8) uint64_t words[3];  // the barrier, the TMEM address, finish()'s barrier
+  for (uint32_t i = threadIdx.x; i < sizeof(rows) / 8; i += TILE) reinterpret_cast<uint64_t *>(rows)[i] = 0;
+  const uint32_t bar = smem_addr(words);
+  if (threadIdx.x < 32) tmem_alloc<32>(bar + 8);
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  fence_smem();
   fence_before();
   __syncthreads();
-  if (threadIdx.x < 32) {
-    fence_after();
-    tmem_free<512>(Group::tmem());
-  }
+  fence_after();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&words[1]);
+  if (threadIdx.x == 0)
+    mma(tmem, operand(smem_addr(rows), TILE * 16), operand(smem_addr(rows) + TILE * 32, Y_COLS * 16), idesc(Y_COLS), false);
+  __syncwarp();
+  uint32_t phase = 0;
+  mbar_wait(bar, phase, &d_expired, polls);
+  finish<32>(tmem, phase, bar + 16, threadIdx.x == 0, 1, &d_expired);
 }
 
 }  // namespace tc

@@ -320,6 +320,10 @@ __device__ __forceinline__ void permutation(uint64_t s[WIDTH]) {
   for (int i = 0; i < WIDTH; i++) s[i] = canon(s[i]);
 }
 
+// Bounded waits that gave up on this device since the library was loaded: of the tensor-core kernels
+// (the NTT's too, which get the address) and of the fused batch.
+__device__ unsigned long long d_expired;
+
 }  // namespace glc
 #include "p2_spread.cuh"
 #include "p2_tensor.cuh"
@@ -420,7 +424,7 @@ __global__ void __launch_bounds__(tc::TILE *tc::GROUPS, 1)
       for (int k = 0; k < 4; k++) results[i + k * count] = store_intermediate ? s[8 + k] : s[k];
     }
   }
-  tc::teardown();
+  tc::teardown(g);
 }
 
 // Node hashes (poseidon2_gl_st.cu:61-82): node i = P2(L0..L3, R0..R3, 0,0,0,0)[0..4] with
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(tc::TILE *tc::GROUPS, 1)
       for (int k = 0; k < 4; k++) results[k * count + gid] = s[k];
     }
   }
-  tc::teardown();
+  tc::teardown(g);
 }
 
 // gather_rows (queries.cuh:9-19)
@@ -663,6 +667,8 @@ int p2_tree_nodes_launch(uint64_t *layer0, uint64_t leaves, uint32_t layers, cud
   return 0;
 }
 
+int expired_counter(unsigned long long **out) { return (int)cudaGetSymbolAddress(reinterpret_cast<void **>(out), d_expired); }
+
 int p2_install_round_constants(const uint64_t *rc) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -696,6 +702,20 @@ bool p2_constants_installed() {
 }  // namespace glc
 
 using namespace glc;
+
+extern "C" glc_status glc_expired_waits(uint64_t *out) {
+  if (!out) return fail("expired_waits: null output");
+  unsigned long long v = 0;
+  const cudaError_t e = cudaMemcpyFromSymbol(&v, d_expired, sizeof(v));
+  *out = v;
+  return (int)e;
+}
+
+extern "C" glc_status glc_expired_wait_probe(uint32_t polls, void *stream) {
+  if (polls > tc::WAIT_POLLS) return fail("expired_wait_probe: at most 50000 polls");
+  tc::expired_wait_kernel<<<1, tc::TILE, 0, (cudaStream_t)stream>>>(polls);
+  return last_launch_error();
+}
 
 extern "C" glc_status glc_poseidon2_set_round_constants(const uint64_t *round_constants) {
   if (!round_constants) return fail("poseidon2: null round constants");

@@ -46,6 +46,7 @@ struct Request {
   bool started = false, done = false, cancelled = false;
   int stream = -1;
   cudaEvent_t done_event = nullptr;
+  uint64_t expired_before = 0;  // a count of given-up waits from before its kernels
   uint64_t *d_evals = nullptr, *d_lde = nullptr, *d_trees = nullptr, *d_cap = nullptr;
 };
 
@@ -58,6 +59,11 @@ struct Server {
   uint32_t classes = 1;
   cudaStream_t copy_stream = nullptr;  // result copies to the host
   cudaMemPool_t pool = nullptr;        // private stream-ordered pool (release threshold: never)
+  // the device's count of waits that gave up (glc_expired_waits): where it is, a page-locked word its
+  // copies arrive in, and the last one seen (worker thread only)
+  const unsigned long long *expired_counter = nullptr;
+  uint64_t *expired_word = nullptr;
+  uint64_t expired_seen = 0;
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
   std::deque<uint64_t> pending;
@@ -121,6 +127,7 @@ static int start_request(Server &s, Request &q) {
   const uint64_t n = 1ull << r.log_n, f = 1ull << r.log_lde;
   cudaStream_t st = s.streams[q.stream];
   cudaError_t e = cudaSuccess;
+  q.expired_before = s.expired_seen;
   // The pool keeps freed blocks mapped (release threshold: never), so requests of other sizes can
   // find the device full of cached blocks they cannot use.  On an allocation failure the pool
   // gives those blocks back (trim) and the allocation is retried; if that is not enough, the
@@ -179,12 +186,19 @@ static void free_request(Server &s, Request &q, bool keep_resident) {
 }
 
 // Copies the cap of a finished request to the host and frees its buffers (worker thread, lock
-// NOT held).  Returns the request's final status.
+// NOT held).  Returns the request's final status: an error when a wait of some kernel on the device gave
+// up since the request was admitted or the last one before it finished, as its results may be wrong.
 static int finish_request(Server &s, Request &q, int status) {
   if (!status) {
     cudaError_t ce = cudaMemcpyAsync(q.req.host_cap, q.d_cap, (4ull << q.req.log_cap) * 8, cudaMemcpyDeviceToHost,
                                      s.copy_stream);
+    if (ce == cudaSuccess)
+      ce = cudaMemcpyAsync(s.expired_word, s.expired_counter, sizeof(uint64_t), cudaMemcpyDeviceToHost, s.copy_stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s.copy_stream);
+    if (ce == cudaSuccess) {
+      s.expired_seen = *s.expired_word;
+      if (s.expired_seen != q.expired_before) ce = cudaErrorTimeout;
+    }
     status = (int)ce;
   }
   free_request(s, q, q.req.keep_resident && !status);
@@ -303,6 +317,16 @@ extern "C" glc_status glc_server_create(const glc_server_config *config, glc_ser
     delete srv;
     return fail("serve: cannot create the copy stream");
   }
+  s.expired_counter = current_tables()->expired;
+  pe = cudaHostAlloc((void **)&s.expired_word, sizeof(uint64_t), cudaHostAllocDefault);
+  int we = pe != cudaSuccess ? (int)pe : glc_expired_waits(&s.expired_seen);
+  if (we) {
+    if (s.expired_word) cudaFreeHost(s.expired_word);
+    cudaStreamDestroy(s.copy_stream);
+    cudaMemPoolDestroy(s.pool);
+    delete srv;
+    return we;
+  }
   // stream priorities: up to 4 classes from the device's range (greatest is numerically lowest)
   int least = 0, greatest = 0;
   if (!s.cfg.flat_priority && cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess)
@@ -315,6 +339,7 @@ extern "C" glc_status glc_server_create(const glc_server_config *config, glc_ser
                                         : cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
       for (auto x : s.streams) cudaStreamDestroy(x);
+      cudaFreeHost(s.expired_word);
       cudaStreamDestroy(s.copy_stream);
       cudaMemPoolDestroy(s.pool);
       delete srv;
@@ -443,6 +468,7 @@ extern "C" glc_status glc_server_destroy(glc_server *srv) {
     cudaStreamDestroy(st);
   }
   if (s.copy_stream) cudaStreamDestroy(s.copy_stream);
+  if (s.expired_word) cudaFreeHost(s.expired_word);
   if (s.pool) cudaMemPoolDestroy(s.pool);  // every block was freed above (stream-ordered, synchronised)
   delete srv;
   return 0;

@@ -77,13 +77,15 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
-// Waits for the barrier's current phase: bounded (about a second).  `phase` bit 0 is the phase's
-// parity, bit 1 records that a wait gave up, after which later waits poll once.  Returns false on
-// the wait that gave up, so that the caller can count it; the kernel then runs to its end with
-// wrong results.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t &phase) {
+// Waits for the barrier's current phase: bounded (`polls` of up to 20 us, about a second).  `phase` bit
+// 0 is the phase's parity, bit 1 records that a wait gave up, after which later waits poll once.  Every
+// thread has a limit of its own, and each whose wait gave up counts itself in *expired; the kernel then
+// runs to its end with wrong results, and finish() below waits for what it left in flight.
+static constexpr uint32_t WAIT_POLLS = 50000;
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t &phase, unsigned long long *expired,
+                                          uint32_t polls = WAIT_POLLS) {
   uint32_t done = 0;
-  for (uint32_t tries = 0; tries < 50000; tries++) {
+  for (uint32_t tries = 0; tries < polls; tries++) {
     asm volatile("{\n\t.reg .pred p;\n\t"
                  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}"
@@ -93,9 +95,35 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t &phase) {
     if (done || (phase >> 1)) break;
   }
   phase ^= 1u;
-  if (!done) phase |= 2u;
+  if (!done) {
+    phase |= 2u;
+    atomicAdd(expired, 1ull);
+  }
   fence_after();
-  return done != 0;
+}
+
+// The CTA's end: frees its TMEM (by warp 0).  After a wait that gave up, products may still read the
+// operand rows and write the TMEM: the threads that issued them (`issuer`, `issuers` of them) then
+// commit once more, to the unused barrier `drain`, and everyone waits for that, bounded, first.
+template <uint32_t COLUMNS>
+__device__ __forceinline__ void finish(uint32_t tmem, uint32_t phase, uint32_t drain, bool issuer, uint32_t issuers,
+                                       unsigned long long *expired) {
+  fence_before();
+  if (__syncthreads_or(phase >> 1)) {
+    if (threadIdx.x == 0) mbar_init(drain, issuers);
+    fence_smem();
+    __syncthreads();
+    if (issuer) commit(drain);
+    __syncwarp();
+    uint32_t last = 0;
+    mbar_wait(drain, last, expired);
+    fence_before();
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+    fence_after();
+    tmem_free<COLUMNS>(tmem);
+  }
 }
 
 // The field element with these 8 digit sums (each at most digit_limit), in [0, 2^64).  Pairs of

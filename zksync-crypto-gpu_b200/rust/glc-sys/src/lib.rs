@@ -175,6 +175,8 @@ extern "C" {
     pub fn glc_mapped_word_create(host: *mut *mut u32, device: *mut *mut u32) -> GlcStatus;
     pub fn glc_mapped_word_destroy(host: *mut u32) -> GlcStatus;
     pub fn glc_commit_batch_fused_timeouts(out: *mut u64) -> GlcStatus;
+    pub fn glc_expired_waits(out: *mut u64) -> GlcStatus;
+    pub fn glc_expired_wait_probe(polls: u32, stream: Stream) -> GlcStatus;
     pub fn glc_commit_graph_create(jobs: *const glc_commit_job, n_jobs: u32, n_streams: u32,
         out: *mut *mut glc_graph) -> GlcStatus;
     pub fn glc_commit_graph_launch(graph: *mut glc_graph, stream: Stream) -> GlcStatus;
