@@ -1,6 +1,6 @@
 """Leaf and node hashing with the partial rounds on the tensor cores (from 2^18 leaves or nodes on),
 against the oracle: partial tiles, rows per leaf, checkpoints, installed round constants, commitments
-alone and in a batch."""
+alone and in a batch, calls that follow the installation of their tables at once."""
 import numpy as np
 import pytest
 
@@ -57,6 +57,33 @@ def test_installed_constants(glc, oracle, round_constants):
         oracle.set_round_constants(other)
         glc.GLHasher.compute_leaf_hashes(to_dev(x), out, 0, False, False)
         assert (from_dev(out) == oracle.leaves(x, 4 * N)).all()
+    finally:
+        glc.poseidon2.set_round_constants(round_constants)
+        oracle.set_round_constants(round_constants)
+
+
+def test_tables_are_there_when_the_call_returns(glc, oracle, round_constants):
+    """Work enqueued at once on a non-blocking stream, which waits for no copy that is still under way."""
+    import torch
+    x, y = rand_elems(8 * N, 3), rand_elems(N, 4)
+    d, side = to_dev(x), torch.cuda.Stream()
+    out, ntt = zeros_dev(4 * N), zeros_dev(4 * N)
+    want = oracle.batch_ntt(y, 18, 1, N, N, 0, 1, 0, 0)
+    try:
+        for seed in range(3):
+            other = [int(v) for v in rand_elems(360, 20 + seed)]
+            oracle.set_round_constants(other)
+            ntt.copy_(to_dev(np.tile(y, 4)))
+            torch.cuda.synchronize()
+            glc.Context.create()
+            with torch.cuda.stream(side):
+                glc.ntt.batch_ntt_in_place(ntt, 18, 4, 0, N, False, True, 0, 0)
+            glc.poseidon2.set_round_constants(other)
+            with torch.cuda.stream(side):
+                glc.GLHasher.compute_node_hashes(d, out)
+            side.synchronize()
+            assert (from_dev(out) == oracle.nodes(x)).all()
+            assert (from_dev(ntt).reshape(4, N) == want).all()
     finally:
         glc.poseidon2.set_round_constants(round_constants)
         oracle.set_round_constants(round_constants)

@@ -114,10 +114,12 @@ extern "C" glc_status glc_context_create(uint32_t powers_of_w_coarse_log_count, 
                                                                        (uint32_t)tw_count);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = (cudaError_t)ntt_init_device();
   if (e == cudaSuccess) e = (cudaError_t)ntt_dft_create(&t.dft);
   if (e == cudaSuccess) e = (cudaError_t)expired_counter(&t.expired);
+  // after every table: a copy from pageable memory may return before it has arrived, and a non-blocking
+  // stream would not wait for it
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     free_tables(t);
     return (int)e;

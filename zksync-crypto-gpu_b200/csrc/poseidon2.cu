@@ -689,6 +689,8 @@ int p2_install_round_constants(const uint64_t *rc) {
     const tc::Matrices m = tc::make_matrices(t);
     e = cudaMemcpyToSymbol(tc::d_matrices, &m, sizeof(m));
   }
+  // the copies may return before they have arrived, and a non-blocking stream would not wait for them
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e == cudaSuccess && dev >= 0 && dev < MAX_DEVICES) g_rc_installed[dev] = true;
   return (int)e;
 }
