@@ -1,6 +1,7 @@
 """Small launches may begin before the previous kernel of their stream has ended (they wait for it
 inside): chains of dependent calls, with other kernels between them, on a side stream and replayed
-from a captured graph, give what the calls one at a time give."""
+from a captured graph, give what the calls one at a time give.  Launches of 74, 148 and more CTAs, and
+transforms of which one pass is small enough to begin early and the other is not."""
 import numpy as np
 import pytest
 
@@ -31,7 +32,8 @@ def chain(glc, d, log_n, cols, n, other=False):
         glc.ntt.batch_ntt_in_place(d, log_n, cols, 0, n, True, True, 1, 1)
 
 
-@pytest.mark.parametrize("log_n,cols", [(1, 1), (9, 3), (10, 5), (13, 2), (16, 1)])
+@pytest.mark.parametrize("log_n,cols", [(1, 1), (9, 3), (10, 5), (10, 148), (10, 149), (13, 2), (13, 8), (16, 1), (16, 2),
+                                        (17, 1), (17, 2)])
 def test_chains(glc, oracle, log_n, cols):
     T = torch()
     n = 1 << log_n

@@ -212,12 +212,14 @@ int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_n
         b.out += (uint64_t)y0 * cpc * b.out_stride;
         b.num_cols = std::min<uint32_t>(cols - y0 * cpc, ycount * cpc);
         const dim3 grid((uint32_t)tiles_per_col, ycount);
+        b.early = launches_early(grid);
+        const size_t bytes = b.early ? std::max(smem, EARLY_SMEM) : smem;
         if (tu.radix_bits == 2)
-          launch(ntt_pass_kernel<2>, grid, threads, smem, stream, b);
+          launch(ntt_pass_kernel<2>, grid, threads, bytes, stream, b);
         else if (tu.radix_bits == 4)
-          launch(ntt_pass_kernel<4>, grid, threads, smem, stream, b);
+          launch(ntt_pass_kernel<4>, grid, threads, bytes, stream, b);
         else
-          launch(ntt_pass_kernel<3>, grid, threads, smem, stream, b);
+          launch(ntt_pass_kernel<3>, grid, threads, bytes, stream, b);
       }
       const int e = last_launch_error();
       if (e) return e;

@@ -36,6 +36,7 @@ struct PassArgs {
                       // coset factor on load, no coset factor on store
   uint32_t j_bitrev;  // exponent j = bitrev_L(position) instead of position
   uint32_t log_ext, coset;
+  uint32_t early;     // launched early: waits for the previous kernel and lets the next one begin
   uint64_t n_inv;
   const uint64_t *g_lo, *g_hi;  // powers of g (scale 1) or g^-1 (scale 2)
   const uint64_t *w_lo, *w_hi;  // powers of w_{2^30}
@@ -175,7 +176,7 @@ __device__ __forceinline__ void ntt_pass_tile(const PassArgs &a, uint32_t bx, ui
     for (uint32_t w = threadIdx.x; w < nq; w += blockDim.x)
       Qt[w] = coset_power(a, a.j_bitrev ? brev_low(hi, a.log_n - k) : lo0 + w);
   }
-  dependency_wait();  // the tables above are the context's
+  if (a.early) dependency_wait();  // the tables above are the context's
   const uint32_t col0 = by * a.cols_per_cta;
   const uint32_t col1 = min(col0 + a.cols_per_cta, a.num_cols);
   const uint32_t wmask = (1u << log_w) - 1;
