@@ -1,6 +1,7 @@
 """The NTT passes on the tensor cores against the oracle: every split of the stages into rounds,
 column groups with remainders, in place and out of place, offsets and strides that forbid the wide
-stores, at and just above the sizes from which batches take this path."""
+stores, at and just above the sizes from which batches take this path, and on both sides of those between
+which 2^16 and 2^17 rows leave it."""
 import numpy as np
 import pytest
 
@@ -18,8 +19,10 @@ def glc():
     ctx.destroy()
 
 
-@pytest.mark.parametrize("log_n,cols", [(12, 256), (12, 513), (12, 5000), (16, 16), (16, 67), (17, 16), (18, 8), (19, 5),
-                                        (20, 2), (21, 1), (22, 1), (23, 1), (24, 16)])
+@pytest.mark.parametrize("log_n,cols", [(12, 256), (12, 513), (12, 5000), (16, 16), (16, 19), (16, 20), (16, 21),
+                                        (16, 26), (16, 27), (16, 67), (17, 8), (17, 9), (17, 10), (17, 11), (17, 13),
+                                        (17, 14), (17, 16), (18, 8), (19, 5), (20, 2), (21, 1), (22, 1), (23, 1), (23, 2),
+                                        (24, 16)])
 @pytest.mark.parametrize("bitrev,inverse,log_ext,coset", [(False, False, 0, 0), (False, True, 0, 0), (True, False, 0, 0),
                                                           (True, True, 0, 0), (False, False, 3, 5)])
 def test_against_oracle(glc, oracle, log_n, cols, bitrev, inverse, log_ext, coset):

@@ -155,11 +155,24 @@ NttTuning &ntt_tuning(uint32_t log_n) {
 // matrices and twiddles cost more to build.  Measured on B200, us, tensor cores / radix passes:
 //   no coset: 16 x 2^16 (256 tiles) 30 / 30, 4 x 2^18 33 / 36, 1 x 2^20 34 / 40; 8 x 2^16 (128) 23 / 22
 //   coset:    32 x 2^16 (512 tiles) 47 / 53, 8 x 2^18 52 / 61; 16 x 2^16 (256) 36 / 32, 4 x 2^18 39 / 38
-//   2^24, whose strided rows hold one element: 1 column 636 / 565, 16 columns 7761 / 8482
+//   2^24, whose strided rows hold one element: 1 column 636 / 565, 16 columns 7761 / 8482; of two: 2^23 on a
+//   coset, 1 column 280 / 257, 2 columns 408 / 457
+// More tiles than the 296 CTAs of a wave take two columns a CTA, and the time of a second column before
+// there are enough of them.  2^16 and 2^17 rows, whose radix passes are the quickest, wait for that:
+//   n2b: 19 x 2^16 (304 tiles) 31 / 33, 20 x 2^16 39 / 34, 25 x 2^16 (400) 39 / 39, 26 x 2^16 39 / 43,
+//        10 x 2^17 (320) 45 / 37, 13 x 2^17 (416) 45 / 43, 14 x 2^17 (448) 45 / 47
+//   b2n inverse: 10 x 2^17 41 / 38, 20 x 2^16 36 / 35, 21 x 2^16 (336) 36 / 38
+//   exactly 256 tiles, n2b forward: 16 x 2^16 28.8 / 26.8, 8 x 2^17 30.9 / 29.4 (the other way no slower)
+//   but 5 and 7 x 2^18 (320, 448) 35 / 43, 45 / 55
 static bool tt_usable(uint32_t log_n, uint32_t num_ntts, bool bitrev_inputs, bool inverse, uint32_t log_ext) {
   if (log_n < TT_LOG || (log_n > TT_LOG && log_n < TT_LOG + 4) || (log_ext && (inverse || bitrev_inputs))) return false;
-  if (log_n == 24 && num_ntts < 16) return false;
-  return ((uint64_t)num_ntts << (log_n - TT_LOG)) >= (log_ext ? 512 : 256);
+  if ((log_n == 24 && num_ntts < 16) || (log_n == 23 && log_ext && num_ntts < 2)) return false;
+  const uint64_t tiles = (uint64_t)num_ntts << (log_n - TT_LOG);
+  if ((log_n == 16 || log_n == 17) && !log_ext) {
+    if (tiles > 304 && tiles < (bitrev_inputs ? 336 : log_n == 16 ? 416 : 432)) return false;
+    if (tiles == 256 && !bitrev_inputs && !inverse) return false;
+  }
+  return tiles >= (log_ext ? 512 : 256);
 }
 
 int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_ntts, uint64_t in_stride,
