@@ -89,15 +89,19 @@ def test_tables_are_there_when_the_call_returns(glc, oracle, round_constants):
         oracle.set_round_constants(round_constants)
 
 
-def test_commitment_alone_and_in_a_batch(glc, oracle):
-    log_n, cols, log_lde, log_cap = 18, 9, 1, 4
+@pytest.mark.parametrize("log_n,cols", [(11, 8), (12, 9), (13, 3), (18, 9)])
+def test_commitment_alone_and_in_a_batch(glc, oracle, log_n, cols):
+    """The leaves' form follows what hashes beside them: nothing, the other coset, other jobs."""
+    log_lde, log_cap = 1, 4
     ev = rand_elems(cols << log_n, 5)
     _, lde, trees, cap = oracle.commit(ev, log_n, cols, log_lde, log_cap)
     sz = glc.CommitJob.sizes(log_n, cols, log_lde, log_cap)
     jobs = [glc.CommitJob(to_dev(ev), log_n, cols, log_lde, log_cap, zeros_dev(sz["lde"]), zeros_dev(sz["trees"]),
-                          zeros_dev(sz["cap"])) for _ in range(3)]
+                          zeros_dev(sz["cap"])) for _ in range(6)]
     glc.commit.commit(jobs[0])
-    glc.commit.commit_batch(jobs[1:])
+    glc.commit.commit_batch(jobs[1:2])
+    glc.commit.commit_batch(jobs[2:4])
+    glc.commit.commit_batch(jobs[4:], n_streams=1)
     for j in jobs:
         assert (from_dev(j.cap) == cap).all()
         assert (from_dev(j.trees) == trees).all()

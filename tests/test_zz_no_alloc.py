@@ -46,8 +46,8 @@ def _cap_noalloc(glc, ev_dev, log_n, cols, log_lde, log_cap):
 
 
 # (log_n, cols, log_lde, log_cap): two ordinary shapes, the exact limit 2^0 * (248 + 8) * 2^16 =
-# 2^24 (the monomials sit in place in coset 0), and LDE x16
-SHAPES = [(14, 64, 1, 4), (13, 40, 2, 4), (16, 248, 0, 4), (12, 8, 4, 4)]
+# 2^24 (the monomials sit in place in coset 0), LDE x16, and leaves that fill the GPU
+SHAPES = [(14, 64, 1, 4), (13, 40, 2, 4), (16, 248, 0, 4), (12, 8, 4, 4), (18, 24, 0, 4)]
 
 
 def test_noalloc_cap_equals_commit_cap_and_oracle(glc, syn, oracle):

@@ -154,7 +154,7 @@ extern "C" glc_status glc_autotune(uint32_t log_n_min, uint32_t log_n_max, uint3
         c.min_blocks = minb;
         p2_tuning() = c;
         const float ms = time_ms(s, (int)reps, [&] {
-          return p2_leaves_launch(buf, buf + LEAF_COLS * count, 0, LEAF_COLS, count, false, false, s, ~0ull);
+          return p2_leaves_launch(buf, buf + LEAF_COLS * count, 0, LEAF_COLS, count, false, false, s, Beside{MANY_LEAVES, true});
         }, &err);
         if (err) break;
         if (ms < best_ms) {

@@ -80,13 +80,15 @@ static int coset_streams_get(uint32_t n, CosetStreams **out) {
   return 0;
 }
 
-int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *events, bool coset_parallel) {
+int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *events, bool coset_parallel, bool shared,
+                   bool yields) {
   uint32_t ev = 0;
   cudaStream_t cur = stream;
   auto mark = [&]() -> int { return events ? (int)cudaEventRecord(events[ev++], cur) : 0; };
   const uint64_t n = 1ull << j.log_n;
   const uint32_t f = 1u << j.log_lde;
   const uint64_t coset_elems = n * j.cols;
+  const Beside beside{shared ? MANY_LEAVES : coset_parallel ? f * n : n, yields};
   // monomials: the caller's buffer, or the last coset's LDE buffer (transformed last, in place)
   uint64_t *mono = j.monomials ? j.monomials : j.lde + (uint64_t)(f - 1) * coset_elems;
   int e = mark();
@@ -125,7 +127,7 @@ int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *ev
     if (!e) e = mark();
     if (e) return e;
     uint64_t *tree = j.trees + (uint64_t)c * 8 * n;
-    e = p2_leaves_launch(dst, tree, 0, j.cols, n, false, false, cur, coset_parallel ? f * n : ~0ull);
+    e = p2_leaves_launch(dst, tree, 0, j.cols, n, false, false, cur, beside);
     if (!e) e = mark();
     if (e) return e;
     if (layers > 1) {
@@ -158,7 +160,7 @@ extern "C" glc_status glc_commit_profiled(const glc_commit_job *job, void *strea
   if (e) return e;
   if (n_events < 3 + 4 * (1u << job->log_lde)) return fail("commit: need 3 + 4 * 2^log_lde events");
   if (!current_tables()) return fail("commit: glc_context_create has not been called on this device");
-  return commit_enqueue(*job, (cudaStream_t)stream, reinterpret_cast<cudaEvent_t *>(events), true);
+  return commit_enqueue(*job, (cudaStream_t)stream, reinterpret_cast<cudaEvent_t *>(events), true, false, false);
 }
 
 extern "C" glc_status glc_commit(const glc_commit_job *job, void *stream) {
@@ -166,5 +168,5 @@ extern "C" glc_status glc_commit(const glc_commit_job *job, void *stream) {
   int e = commit_check(*job);
   if (e) return e;
   if (!current_tables()) return fail("commit: glc_context_create has not been called on this device");
-  return commit_enqueue(*job, (cudaStream_t)stream, nullptr, true);
+  return commit_enqueue(*job, (cudaStream_t)stream, nullptr, true, false, false);
 }

@@ -82,10 +82,15 @@ int ntt_launch(const uint64_t *in, uint64_t *out, uint32_t log_n, uint32_t num_n
                cudaStream_t stream, uint32_t l2_chunk_cols, bool registers_only = false);
 int bitrev_launch(const uint64_t *src, uint64_t src_stride, uint64_t *dst, uint64_t dst_stride, uint32_t log_rows,
                   uint32_t cols, cudaStream_t stream);
-// together: leaves that other streams hash at the same time, these included (a launch that shares the
-// GPU takes the form that needs the fewest instructions, not the shortest chain).
+// What hashes beside a launch.
+struct Beside {
+  uint64_t leaves = 0;  // leaves hashed at the same time, the launch's own included (few: the form with the
+                        // shortest chain, many: the one that needs the fewest instructions)
+  bool yields = false;  // launches of higher priority may arrive: no CTAs that keep an SM to the launch's end
+};
+static constexpr uint64_t MANY_LEAVES = ~0ull;
 int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t rows, uint64_t cols, uint64_t count,
-                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, uint64_t together = 0);
+                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, Beside beside = {});
 int p2_nodes_launch(const uint64_t *values, uint64_t *results, uint64_t count, cudaStream_t stream);
 // Node layers of a tree whose leaf layer ([4][leaves]) starts at `layer0`; writes layers 1..layers
 // into the following part of the same buffer (reference layout, poseidon2.rs:276-314).
@@ -103,7 +108,8 @@ int commit_check(const glc_commit_job &j);
 // runs the coset, then one after the cap gather (3 + 4 * 2^log_lde events).
 // coset_parallel: run the cosets on internal streams forked from `stream` (one call); the batch
 // and serving runtimes pass false because they already spread jobs over streams.
-int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *events = nullptr,
-                   bool coset_parallel = false);
+// shared: other jobs run beside this one; yields: as in Beside.
+int commit_enqueue(const glc_commit_job &j, cudaStream_t stream, cudaEvent_t *events, bool coset_parallel, bool shared,
+                   bool yields);
 
 }  // namespace glc

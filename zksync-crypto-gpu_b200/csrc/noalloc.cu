@@ -94,5 +94,5 @@ extern "C" glc_status glc_commit_cap_noalloc(const uint64_t *evals, uint64_t eva
   j.lde = scratch;                              // f cosets x cols x 2^log_n
   j.trees = scratch + f * (uint64_t)cols * n;   // f subtrees x 8 x 2^log_n
   j.monomials = nullptr;                        // kept in the last coset's LDE slot
-  return commit_enqueue(j, (cudaStream_t)stream, nullptr, false);
+  return commit_enqueue(j, (cudaStream_t)stream, nullptr, false, false, false);
 }

@@ -567,11 +567,17 @@ static void leaves_go(uint32_t minb, uint32_t blocks, uint32_t threads, cudaStre
 // 16384: 50 / 25.8 / 21.7.
 static constexpr uint64_t HEX_MAX = 2048, QUAD_MAX = 8192;
 
-// From this many leaves or nodes on, a launch runs its partial rounds on the tensor cores (p2_tensor.cuh),
-// unless it shares the GPU with other jobs' small kernels, which its CTAs, one to an SM, would keep
-// out.  Measured on B200, G permutations/s, tensor / a thread each: nodes 2^16 1.25 / 1.20, 2^17 1.50 /
-// 1.49, 2^18 1.67 / 1.56, 2^22 1.77 / 1.66; leaves of 32 columns 2^16 1.42 / 1.35, 2^17 1.59 / 1.58,
-// 2^18 1.71 / 1.62; of 176 columns 2^15 1.16 / 1.28, 2^22 1.75 / 1.69.
+// From this many leaves or nodes on, a launch runs its partial rounds on the tensor cores (p2_tensor.cuh).
+// Measured on B200, G permutations/s, tensor / a thread each: nodes 2^16 1.29 / 1.23, 2^17 1.52 / 1.52,
+// 2^18 1.68 / 1.54, 2^22 1.77 / 1.66; leaves of 32 columns 2^16 1.42 / 1.35, 2^17 1.57 / 1.59, 2^18
+// 1.70 / 1.61; of 176 columns 2^15 1.16 / 1.28, 2^22 1.75 / 1.69.  Below 2^18 a launch beside the other
+// coset's leaves is mostly better off without CTAs that take whole SMs: with 2^16 as the line a commitment
+// of 2^18 x 32 takes 2175 us instead of 2119, and one of 2^16 x 32 673 instead of 703.
+// Leaves that must yield (a server's) keep a thread each whatever their number: the CTAs stay to the end
+// of their launch, 53 ms for 176 columns at 2^22, and a smaller request of higher priority would wait for
+// them; a node layer, 2.4 ms at most, does not yield.  Beside other jobs of a batch the tensor cores are
+// the faster form: 8 jobs of 2^18 .. 2^20 rows on streams 108.5 -> 106.3 ms, 300 of 2^12 .. 2^22 4098 ->
+// 4009 (one call per job 4025).
 static constexpr uint64_t TENSOR_MIN = 1 << 18;
 
 // One CTA per SM hashes it all: with CTAs of two tiles a group instead, a CTA's last group and the next
@@ -593,9 +599,9 @@ static uint32_t spread_grid(uint64_t count, uint32_t lanes) {
 }
 
 int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_rows, uint64_t cols, uint64_t count,
-                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, uint64_t together) {
+                     bool load_intermediate, bool store_intermediate, cudaStream_t stream, Beside beside) {
   if (count == 0) return 0;
-  together = std::max(together, count);
+  const uint64_t together = std::max(beside.leaves, count);
   if (together <= QUAD_MAX) {
     if (together <= HEX_MAX)
       p2_leaves_spread_kernel<16><<<spread_grid(count, 16), SPREAD_THREADS, 0, stream>>>(
@@ -605,7 +611,7 @@ int p2_leaves_launch(const uint64_t *values, uint64_t *results, uint32_t log_row
           values, results, log_rows, cols, count, load_intermediate, store_intermediate);
     return last_launch_error();
   }
-  if (count >= TENSOR_MIN && together != ~0ull && cols && (cols << log_rows) <= 0xfffffff0u) {
+  if (count >= TENSOR_MIN && !beside.yields && cols && (cols << log_rows) <= 0xfffffff0u) {
     return tensor_launch(p2_leaves_tensor_kernel, count, stream, values, results, log_rows, (uint32_t)(cols << log_rows),
                          count, load_intermediate, store_intermediate);
   }

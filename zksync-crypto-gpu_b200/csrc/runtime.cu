@@ -94,7 +94,7 @@ int commit_batch_enqueue(const glc_commit_job *jobs, uint32_t n_jobs, uint32_t n
   for (size_t k = 0; k < max_len; k++)
     for (uint32_t s = 0; s < n_streams; s++)
       if (k < assign[s].size()) {
-        e = commit_enqueue(jobs[assign[s][k]], pool->streams[s]);
+        e = commit_enqueue(jobs[assign[s][k]], pool->streams[s], nullptr, false, n_streams > 1, false);
         if (e) return e;
       }
   for (uint32_t s = 0; s < n_streams; s++) {

@@ -162,7 +162,7 @@ static int start_request(Server &s, Request &q) {
     j.lde = q.d_lde;
     j.trees = q.d_trees;
     j.cap = q.d_cap;
-    err = commit_enqueue(j, st);
+    err = commit_enqueue(j, st, nullptr, false, s.inflight > 1, true);
   }
   // the cap goes to the host at completion (worker thread, private copy stream): a copy enqueued
   // here into pageable memory would block this thread until the whole job had finished
