@@ -258,18 +258,20 @@ def test_commit_contract(glc, syn):
 @pytest.mark.parametrize("radix,k1,lw,cpc,mb", [(2, 0, 5, 8, 8), (3, 7, 3, 1, 8), (4, 12, 4, 4, 0), (3, 10, 5, 64, 0),
                                                 (4, 9, 3, 8, 0)])
 def test_ntt_tuning_invariance(glc, oracle, radix, k1, lw, cpc, mb):
-    """Every tuning choice computes the same transform (bit-exact)."""
+    """Every tuning choice computes the same transform (bit-exact).  The transforms are ones that the tuning
+    applies to: a forward n2b coset below 2^21 elements, or a coset on the b2n side or in an inverse."""
     log_n = 20 if k1 != 7 else 14
     n = 1 << log_n
-    cols = 3
     saved = glc.tuning.get_ntt(log_n)
     glc.tuning.set_ntt(log_n, radix, k1, lw, cpc, mb)
     try:
-        x = syn_x = load_synthetic().random_field_elements("tune-%d" % radix, cols * n)
-        for bitrev_inputs, inverse, e, c in ((False, False, 1, 1), (True, True, 2, 3)):
-            d_in, d_out = to_dev(x), zeros_dev(cols * n)
+        x = load_synthetic().random_field_elements("tune-%d" % radix, 3 * n)
+        for cols, bitrev_inputs, inverse, e, c in ((1, False, False, 1, 1), (3, True, False, 1, 1), (3, False, True, 2, 1),
+                                                   (3, True, True, 2, 3)):
+            src = x[:cols * n]
+            d_in, d_out = to_dev(src), zeros_dev(cols * n)
             glc.ntt.batch_ntt_out_of_place(d_in, d_out, log_n, cols, 0, 0, n, n, bitrev_inputs, inverse, e, c)
-            assert (canon(from_dev(d_out)) == oracle.batch_ntt(syn_x, log_n, cols, n, n, bitrev_inputs, inverse, e, c)).all()
+            assert (canon(from_dev(d_out)) == oracle.batch_ntt(src, log_n, cols, n, n, bitrev_inputs, inverse, e, c)).all()
     finally:
         glc.tuning.set_ntt(log_n, saved.radix_bits, saved.k1, saved.max_log_w, saved.max_cols_per_cta, saved.l2_chunk_mb)
 
@@ -278,17 +280,19 @@ def test_ntt_tuning_invariance(glc, oracle, radix, k1, lw, cpc, mb):
                                                      (128, 0, 0, 3), (256, 1, 1, 2), (256, 2, 1, 3), (128, 2, 0, 2),
                                                      (64, 2, 1, 2), (256, 2, 0, 3), (128, 2, 1, 5), (64, 1, 0, 5)])
 def test_leaf_tuning_invariance(glc, oracle, threads, rolled, lazy, minb):
+    """Every tuning choice computes the same digests, at counts that it applies to: above those whose
+    permutations take several lanes each, below those on the tensor cores, for leaves and node layers."""
     saved = glc.tuning.get_p2()
     glc.tuning.set_p2(threads, rolled, lazy, minb)
     try:
-        count, cols = 1 << 10, 11
+        count, cols = 1 << 15, 11
         vals = load_synthetic().random_field_elements("leaf-tune", cols * count)
         d_res = zeros_dev(4 * count)
         glc.GLHasher.compute_leaf_hashes(to_dev(vals), d_res, 0, False, False)
         assert (canon(from_dev(d_res)) == oracle.leaves(vals, 4 * count, 0)).all()
         d_tree = zeros_dev(8 * count)
-        glc.GLHasher.build_merkle_tree(to_dev(vals), d_tree, 0, None, 11)
-        assert (canon(from_dev(d_tree)) == oracle.build_merkle_tree(vals, 8 * count, 0, 11)).all()
+        glc.GLHasher.build_merkle_tree(to_dev(vals), d_tree, 0, None, 16)
+        assert (canon(from_dev(d_tree)) == oracle.build_merkle_tree(vals, 8 * count, 0, 16)).all()
     finally:
         glc.tuning.set_p2(saved.leaf_threads, saved.rolled, saved.lazy, saved.min_blocks)
 
