@@ -427,6 +427,12 @@ def measure_commit(glc, torch, shape, steps, warmup, world, barrier, clocks=None
     return out
 
 
+def leaf_kernel(leaves):
+    """The kernel that hashes this many leaves when no other job runs beside them (csrc/poseidon2.cu)."""
+    return ("p2_leaves_tensor_kernel" if leaves >= 1 << 18 else
+            "p2_leaves_spread_kernel" if leaves <= 8192 else "p2_leaves_kernel")
+
+
 def leaf_alone_ms(glc, torch, job, shape):
     """One coset's leaf launch alone on the stream (in the step it shares the GPU with the other
     coset's kernels, which stretches its duration): median of 3, CUDA events."""
@@ -469,7 +475,8 @@ def run_ours(args, rank, world, local_rank):
     leaf_modmul = MODMUL_PER_PERM * units["perms_leaves"] / f
     achieved = leaf_modmul / (leaf_ms / 1e3) / 1e9
     alone = leaf_alone_ms(glc, torch, job, shape)
-    traffic = facts.get("p2_leaves_kernel_bytes_per_launch_2e22x176")
+    kernel = leaf_kernel(1 << log_n)
+    traffic = facts.get("%s_bytes_per_launch_2e%dx%d" % (kernel, log_n, cols))
     t_roof = max(units["bytes"] / (peaks["hbm_gbs"] * 1e9), units["modmul"] / mm_peak)
     ref = None
     if rank == 0 and not args.no_ref_kernels:
@@ -522,7 +529,7 @@ def run_ours(args, rank, world, local_rank):
                                     frac=max(u["bytes"] / (peaks["hbm_gbs"] * 1e9), u["modmul"] / mm_peak) * 1e3
                                     / max(1e-9, stage[k]))
                             for k, u in stage_units(shape).items()},
-        "roofline": {"bound": "int", "kernel": "p2_leaves_tensor_kernel", "achieved": achieved,
+        "roofline": {"bound": "int", "kernel": kernel, "achieved": achieved,
                      "peak": mm_peak / 1e9, "unit": "Gmodmul/s", "frac": achieved * 1e9 / mm_peak,
                      "launch_ms_in_step": leaf_ms, "launch_ms_alone": alone,
                      "frac_alone": leaf_modmul / (alone / 1e3) / mm_peak,

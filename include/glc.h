@@ -295,8 +295,11 @@ glc_status glc_server_destroy(glc_server *server);
  * them (or autotune) before other host threads launch work on that device.  Every choice
  * computes the same bits.
  */
-/* For the NTT passes in registers; batches large enough for the tensor cores (from 2^20 elements, 2^21
- * on a coset) have a fixed plan. */
+/* For the NTT passes in registers.  Batches that run on the tensor cores have a fixed plan: forward
+ * without a coset and inverse without one from 2^20 elements, forward n2b on a coset from 2^21, at 2^12
+ * and 2^16 .. 2^24 rows, except 2^24 rows below 16 columns, one column of 2^23 on a coset, and at 2^16 and
+ * 2^17 rows the sizes whose tiles end shortly after a wave of CTAs (tt_usable in csrc/ntt.cu).  A coset
+ * with bit-reversed inputs or in an inverse always runs in registers. */
 typedef struct glc_ntt_tuning {
   uint32_t radix_bits;       /* stages per register round: 2, 3 or 4 */
   uint32_t k1;               /* stages in the strided pass of a two-pass NTT (0 = log_n / 2) */
@@ -304,6 +307,9 @@ typedef struct glc_ntt_tuning {
   uint32_t max_cols_per_cta; /* columns one CTA walks with the same twiddles (1..64) */
   uint32_t l2_chunk_mb;      /* a two-pass NTT runs both passes per chunk of this many MiB; 0: one chunk */
 } glc_ntt_tuning;
+/* For leaves and node layers of 8193 .. 2^18 - 1 permutations, and for the leaves of jobs that share the
+ * GPU (other jobs of a batch: up to 2^18 - 1 leaves; a server's: any number).  Fewer permutations take 4 or
+ * 16 lanes each, more the tensor cores. */
 typedef struct glc_p2_tuning {
   uint32_t leaf_threads; /* 64, 128 or 256 (leaf and wide node-layer kernels) */
   uint32_t rolled;       /* 0: fully unrolled, 1: partial rounds in a loop, 2: full rounds too */

@@ -20,7 +20,7 @@
 // are reduced and written.
 //
 // Bound: latency between the rounds of the two CTAs an SM holds (TMEM: 256 of 512 columns each), then
-// the integer pipes (ALU and fmaheavy 45-50%, DRAM 22-39%, tensor 17-20% of peak); the waits for the
+// the integer pipes (ALU and fmaheavy 41-48%, DRAM 21-37%, tensor 10-17% of peak); the waits for the
 // products cost 15%.  About 45 thread instructions per value and round of 4 stages, where the
 // radix-16 register rounds (ntt_tile.cuh) take 104.  Measured on B200, us, register rounds -> this:
 // inverse 2^20 x 128: 2731 -> 1610; 2^22 x 176: 16547 -> 10900; forward coset 2^20 x 128: 2672 -> 1645.

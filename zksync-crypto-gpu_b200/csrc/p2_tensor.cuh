@@ -21,9 +21,9 @@
 // block's four S-box inputs from everything before the block, and the terms inside the block have
 // small coefficients (17, 11, 31718: e_0^T N^m u) and are added directly.
 //
-// Bound: the integer pipes (fmaheavy 72%, ALU 53%) with five warpgroups an SM, as many as the operand
-// rows leave room for in shared memory and one 96-column result each in TMEM; tensor pipe 5%.  A
-// permutation issues 12.2 K instructions, 14.2 K without (the 22 internal layers were 3 K).  Measured
+// Bound: the integer pipes (leaves: fmaheavy 67%, ALU 56%) with five warpgroups an SM, as many as the
+// operand rows leave room for in shared memory and one 96-column result each in TMEM; tensor pipe 4%.  A
+// permutation takes 12.2 K instructions, 14.2 K without (the 22 internal layers were 3 K).  Measured
 // on B200: 2^22 nodes 2532 -> 2365 us, leaves of 176 columns at 2^22 54.6 -> 52.8 ms, registers' worth
 // of addresses kept out of the full rounds included (1.69 -> 1.71 G permutations/s).  Four groups with
 // 128 registers each: 1.68 against 1.78 G permutations/s with five (permutations alone).
